@@ -83,7 +83,7 @@ def parse():
                     help="skip the 64-instance batched ensemble measurement")
     ap.add_argument("--ensemble-steps", type=int, default=10)
     ap.add_argument("--tile-shape", type=int, default=None, choices=[0, 1, 2, 3],
-                    help="particle-kernel tile shape (0 64x4, 1 256x1, 2 128x2, 3 16x16); "
+                    help="particle-kernel tile shape (0 auto, 1 256x1, 2 128x2, 3 16x16); "
                          "default: the library's tuner picks it (under a profiler, fix it: "
                          "the tuner's timings change there)")
     return ap.parse_args()
@@ -397,7 +397,7 @@ def run_ours(args, rank, world, local_rank):
         "warmup": args.warmup, "ms_per_step": part_ms / args.steps, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": {"workload": describe(w), "particles_per_gpu": n_part,
-                   "tile_shape": ["64x4", "256x1", "128x2", "16x16"][tile_shape],
+                   "tile_shape": ["auto", "256x1", "128x2", "16x16"][tile_shape],
                    "ms_per_tile_shape": tile_ms,
                    "particles_per_species": counts, "grid_nodes": (w.nx + 1) * (w.ny + 1),
                    "l2": "inputs larger than L2 (particle state ~%.1f GB per GPU)" % (n_part * 40 / 1e9),
@@ -585,7 +585,7 @@ def run_ensemble(args, rank, world, local_rank):
             "poisson_iters_mean": statistics.mean(m["iters"] for m in every.values()),
             "worst_relres": max(m["relres"] for m in every.values()),
             "push_roofline_frac": BYTES_PUSH_PASS * n_part / world / (push_ms * 1e-3) / 1e9 / peak,
-            "tile_shape": ["64x4", "256x1", "128x2", "16x16"][shape], "ms_per_shape": ms_shapes,
+            "tile_shape": ["auto", "256x1", "128x2", "16x16"][shape], "ms_per_shape": ms_shapes,
             "graph": info["graph"], "solver_blocks": info["solver_blocks"], "steps": args.ensemble_steps,
             "setup_s": setup_s, "scaling": "strong", "n_gpus": world,
             "placement": "whole instances, greedy longest-first on cell counts; rank loads (cells) "

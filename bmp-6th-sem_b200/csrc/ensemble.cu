@@ -47,6 +47,7 @@ struct pic_ensemble {
     bool energy = true;
     bool use_graph = true;
     cudaGraphExec_t graph = nullptr;
+    int graph_kernels = 0;  // batch_kernels() of the captured step
     bool graph_failed = false;
     double last_ms[3] = {0, 0, 0};  // deposit, Poisson (+E), push
 };
@@ -231,12 +232,18 @@ int pic_ensemble_step(pic_ensemble* e, int iteration) {
             if (!c->sp[s].acc_fresh) PIC_TRY(particles_deposit(c, s));
     PIC_TRY(batch_prepare(e->pb, e->cs.data(), e->stream));
     PIC_TRY(upload_poisson(e));
+    const int kernels = batch_kernels(e->pb, e->shape);
+    if (e->graph && e->graph_kernels != kernels) {
+        PIC_CUDA(cudaGraphExecDestroy(e->graph));  // captured with other push kernels
+        e->graph = nullptr;
+    }
     if (e->use_graph && !e->graph && !e->graph_failed) {
         cudaGraph_t g = nullptr;
         bool ok = cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
         const int st = ok ? enqueue_step(e, true) : PIC_ERR_CUDA;
         ok = (cudaStreamEndCapture(e->stream, &g) == cudaSuccess) && ok && st == PIC_OK;
         if (ok) ok = cudaGraphInstantiate(&e->graph, g, 0) == cudaSuccess;
+        e->graph_kernels = kernels;
         if (g) cudaGraphDestroy(g);
         if (!ok) {
             e->graph = nullptr;
@@ -291,10 +298,6 @@ int pic_ensemble_autotune(pic_ensemble* e, int* shape, double* ms_per_shape) {
     int best = 0;
     for (int k = 1; k < nsh; ++k)
         if (ms[k] < ms[best]) best = k;
-    if (best != e->shape && e->graph) {
-        cudaGraphExecDestroy(e->graph);  // captured with the old shape
-        e->graph = nullptr;
-    }
     e->shape = best;
     if (shape) *shape = best;
     if (ms_per_shape)

@@ -15,26 +15,37 @@
 // ones that stayed in the cell at the last push) and a back run (the ones
 // that moved in), with a free gap between them.
 //
-// One push of a species is ONE pass over its particles (k_cells<kPush>): a
-// warp walks a cell, gathers E and Bz, pushes, and
+// One push of a species is ONE pass over its particles (k_cells<kPush>).  A
+// warp works on a few neighbouring cells at a time, 4, 8 or 16 lanes a cell;
+// it gathers E and Bz, pushes, and
 //   * writes a particle that stays in its cell to the front of the cell's
 //     slots in the other buffer, at its rank among the cell's stayers
-//     (ballot + popc: no atomics);
-//   * appends a particle that moves to a neighbouring cell to the back of
-//     that cell's slots: lanes moving the same way form a group
-//     (match.any), the group leader reserves the slots with one atomic on
-//     the target's back count.  The reservation is capped at the target's
-//     capacity minus its current count (the most stayers it can have), so
-//     front and back runs never meet;
-//   * deposits the new position: stayers accumulate per-lane integer
-//     moments reduced once per cell, movers add their four fixed-point
-//     corner weights with 64-bit RED.
-// A mover whose target is full, or which jumped more than one cell, goes to
-// a side list; a small kernel (k_fixup) then places it in the free space of
-// its target cell, or keeps it on the list (still part of the state: it is
-// pushed and deposited from there at the next step).  When the list grows,
-// the host rebuilds the layout from the per-cell counts (k_relayout_*).
-// Per particle-step the HBM traffic is 20 B read + 20 B written.
+//     (ballot + popc: no atomics), and adds its deposit to per-lane integer
+//     sums, reduced once per cell;
+//   * queues a particle that leaves; every 32 of them are placed with all
+//     lanes busy: each reserves a slot at the back of its new cell with one
+//     atomic on the cell's back count, capped at the cell's capacity minus
+//     its current count (the most stayers it can have), so front and back
+//     runs never meet.
+// The deposit of the particles that changed cell is a second, small pass over
+// the back runs (k_cells<kArrivals>): per-cell sums again, where depositing
+// each mover on its own took eight 64-bit REDs.  A mover whose target is full
+// goes to a side list; a small kernel (k_fixup) then deposits it and places
+// it in the free space of its target cell, or keeps it on the list (still
+// part of the state: it is pushed and deposited from there at the next
+// step).  When the list grows, the host rebuilds the layout from the
+// per-cell counts (k_relayout_*).  Per particle-step the HBM traffic is 20 B
+// read + 20 B written.
+//
+// Measured on a B200, push + arrivals, electrons / Ar+: the 1024^2 workload
+// (1.15e8 particles each) 1.26 / 0.88 ms (with a warp a cell, 32-lane chunks
+// and the movers deposited one by one: 1.83 / 1.17 ms); 512^2 at 64 a cell
+// 0.23 / 0.14 ms (0.28 / 0.18); 64 grids of 128^2 .. 384^2 at 32 a cell 4.2 ms
+// both (8.2 ms).  The Ar+ pass runs at 5.2 TB/s of reads and writes, 0.8 of a
+// plain copy; leaving out instructions (the FP32 push, the energy sums)
+// changes it by a few percent, leaving out its stores by 40 %: memory bound.
+// The electrons pay 0.3 ms for placing their 18 % movers (an atomic with its
+// answer, two scattered stores each) and 0.1 ms for the arrivals' pass.
 //
 // Determinism: the charge and energy deposits are sums of integers, so they
 // do not depend on the order in which particles are processed or placed;
@@ -45,6 +56,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "pic_internal.h"
 
@@ -54,7 +66,6 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kThreads = kWarps * 32;
-constexpr int kCellBlocksPerSM = 4;           // k_cells residency (register budget)
 constexpr int kScanTile = 2048;               // cells per scan block
 constexpr uint32_t kAxisOne = 1u << kAxisBits;
 constexpr float kAxisScale = (float)(1u << kAxisBits);
@@ -64,8 +75,7 @@ constexpr float kFloorMagic = 12582912.0f;    // 1.5 * 2^23
 constexpr uint32_t kFloorMagicBits = 0x4B400000u;
 constexpr int kFixupBlocks = 296;
 
-enum Mode { kPush = 0, kDeposit = 1 };
-constexpr int kFar = 9;       // moved more than one cell in x or y
+enum Mode { kPush = 0, kDeposit = 1, kArrivals = 2 };
 
 // list_counts slots
 enum { kOvf = 0, kLoose0 = 1, kLoose1 = 2 };
@@ -112,17 +122,14 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// Asynchronous global -> shared copies (cp.async) to a shared-space address;
-// a false predicate copies nothing and fills the destination with zeros.
+// Asynchronous global -> shared copies (cp.async) to a shared-space address.
 // Only the wait orders them against the shared-memory reads of the data.
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool pred) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src),
-                 "r"(pred ? 16 : 0));
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
 }
 
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, bool pred) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src),
-                 "r"(pred ? 4 : 0));
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src));
 }
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
@@ -139,9 +146,26 @@ struct Pushed {
     int sx, sy;    // cell step: 0, 0 exactly when the particle keeps its cell
     // set by resolve_move
     int gx, gy;
-    int dir;  // 0: moved at most one cell in x and y, kFar: farther, -1: absorbed
-    bool left;
+    bool alive;  // inside the walls
+    bool left;   // absorbed, and through x < 0
 };
+
+// Re-cell of the position (px, py) in units of the old cell: the integer
+// part moves the cell, the remainder is the new offset.  floor without the
+// conversion unit: for |p| < 2^22, p + 1.5*2^23 rounded down is floor(p) +
+// 1.5*2^23 exactly, an integer held in the low mantissa bits; subtracting
+// 1.5*2^23 again is exact.  The step's bits are 0 exactly when floor(p) == 0:
+// for NaN or |p| >= 2^22 the sum is not 1.5*2^23, so those never read as
+// staying.
+__device__ __forceinline__ void recell(Pushed& o) {
+    const float px = o.px, py = o.py;
+    const float tx = __fadd_rd(px, kFloorMagic), ty = __fadd_rd(py, kFloorMagic);
+    const float fsx = __fsub_rn(tx, kFloorMagic), fsy = __fsub_rn(ty, kFloorMagic);
+    o.fx = fminf(__fsub_rn(px, fsx), kOneBelow);
+    o.fy = fminf(__fsub_rn(py, fsy), kOneBelow);
+    o.sx = (int)(__float_as_uint(tx) - kFloorMagicBits);
+    o.sy = (int)(__float_as_uint(ty) - kFloorMagicBits);
+}
 
 // Bilinear gather of E (and Bz) from the cell's four nodes plus the Boris
 // push of deterministic_mover (src/mover.cpp:123-174) in FP32.  Weights:
@@ -151,8 +175,22 @@ struct Pushed {
 //
 // push_move does the arithmetic of every particle; resolve_move the cell
 // bookkeeping that only particles leaving their cell need.
-__device__ __forceinline__ Pushed push_move(float4 a, float4 n00, float4 n10, float4 n01,
-                                            float4 n11, const SpeciesConsts& k) {
+// A node's field: {Ex, Ey}, with Bz (and padding) unless it is uniform.
+template <bool BZU>
+struct __align__(16) NodeField {
+    float x, y, z, w;
+    __device__ __forceinline__ static NodeField from(float4 f) { return NodeField{f.x, f.y, f.z, f.w}; }
+};
+template <>
+struct __align__(8) NodeField<true> {
+    float x, y;
+    static constexpr float z = 0.f;  // not read
+    __device__ __forceinline__ static NodeField from(float4 f) { return NodeField{f.x, f.y}; }
+};
+
+template <bool BZU>
+__device__ __forceinline__ Pushed push_move(float4 a, NodeField<BZU> n00, NodeField<BZU> n10, NodeField<BZU> n01,
+                                            NodeField<BZU> n11, const SpeciesConsts& k) {
     const float fx = a.x, fy = a.y;
     const float ofx = __fsub_rn(1.0f, fx), ofy = __fsub_rn(1.0f, fy);
     const float w00 = __fmul_rn(ofx, ofy), w10 = __fmul_rn(fx, ofy);
@@ -161,7 +199,7 @@ __device__ __forceinline__ Pushed push_move(float4 a, float4 n00, float4 n10, fl
     const float ey = __fmaf_rn(w11, n11.y, __fmaf_rn(w01, n01.y, __fmaf_rn(w10, n10.y, __fmul_rn(w00, n00.y))));
     // Boris rotation about z (src/mover.cpp:151-162): t = h Bz, s = 2t/(1+t^2)
     float t, s;
-    if (k.bzu) {
+    if (BZU) {
         t = k.bt;
         s = k.bs;
     } else {
@@ -177,25 +215,17 @@ __device__ __forceinline__ Pushed push_move(float4 a, float4 n00, float4 n10, fl
     Pushed o;
     o.vx = __fadd_rn(__fmaf_rn(vyp, s, vxm), ax);
     o.vy = __fadd_rn(__fmaf_rn(-vxp, s, vym), ay);
-    // Position update in cell units (src/mover.cpp:164-165), then re-cell:
-    // the integer part moves the cell, the remainder is the new offset.
-    const float px = __fmaf_rn(o.vx, k.dtdx, fx);
-    const float py = __fmaf_rn(o.vy, k.dtdy, fy);
-    o.px = px;
-    o.py = py;
-    // floor without the conversion unit: for |p| < 2^22, p + 1.5*2^23
-    // rounded down is floor(p) + 1.5*2^23 exactly, an integer held in the
-    // low mantissa bits; subtracting 1.5*2^23 again is exact.  The step's
-    // bits are 0 exactly when floor(p) == 0: for NaN or |p| >= 2^22 the sum
-    // is not 1.5*2^23, so those never read as staying.
-    const float tx = __fadd_rd(px, kFloorMagic), ty = __fadd_rd(py, kFloorMagic);
-    const float fsx = __fsub_rn(tx, kFloorMagic), fsy = __fsub_rn(ty, kFloorMagic);
-    o.fx = fminf(__fsub_rn(px, fsx), kOneBelow);
-    o.fy = fminf(__fsub_rn(py, fsy), kOneBelow);
-    o.sx = (int)(__float_as_uint(tx) - kFloorMagicBits);
-    o.sy = (int)(__float_as_uint(ty) - kFloorMagicBits);
+    // Position update in cell units (src/mover.cpp:164-165)
+    o.px = __fmaf_rn(o.vx, k.dtdx, fx);
+    o.py = __fmaf_rn(o.vy, k.dtdy, fy);
     return o;
 }
+
+// 0 <= p < 1, the particle keeps its cell in this axis: as unsigned integers
+// the bits of the floats in [0, 1) are below those of 1 and every other
+// float's (negative ones and NaN included) are not.  (-0 reads as leaving;
+// it is then placed into its own cell again.)  The new offset is p itself.
+__device__ __forceinline__ bool keeps_cell(float p) { return __float_as_uint(p) < 0x3f800000u; }
 
 // Cell bookkeeping of a pushed particle that was in cell (gx, gy).
 __device__ __forceinline__ void resolve_move(Pushed& o, const SpeciesConsts& k, int gx, int gy,
@@ -214,31 +244,34 @@ __device__ __forceinline__ void resolve_move(Pushed& o, const SpeciesConsts& k, 
         if (o.gy < 0) o.gy += ny;
     }
     // absorbing walls (src/mover.cpp:325): outside [0,W) x [0,H)
-    const bool alive = ok && (unsigned)o.gx < (unsigned)nx && (unsigned)o.gy < (unsigned)ny;
+    o.alive = ok && (unsigned)o.gx < (unsigned)nx && (unsigned)o.gy < (unsigned)ny;
     o.left = ok ? (o.gx < 0) : (px < 0.0f);
-    const bool near = (unsigned)(sx + 1) < 3u && (unsigned)(sy + 1) < 3u;
-    o.dir = !alive ? -1 : (near ? 0 : kFar);
 }
 
 __device__ __forceinline__ Pushed push_one(float4 a, float4 n00, float4 n10, float4 n01,
                                            float4 n11, const SpeciesConsts& k, int gx, int gy,
                                            int nx, int ny) {
-    Pushed o = push_move(a, n00, n10, n01, n11, k);
+    using U = NodeField<true>;
+    using V = NodeField<false>;
+    Pushed o = k.bzu ? push_move<true>(a, U::from(n00), U::from(n10), U::from(n01), U::from(n11), k)
+                     : push_move<false>(a, V::from(n00), V::from(n10), V::from(n01), V::from(n11), k);
+    recell(o);
     resolve_move(o, k, gx, gy, nx, ny);
     return o;
 }
 
-// round(f * 2^20) for f in [0, 1): exact scaling, then the 1.5*2^23 addition
-// rounds to nearest-even in the mantissa (integer ALU, no conversion unit).
+// round(f * 2^20) for f in [0, 1): the scaling is exact, so one FMA with
+// 1.5*2^23 rounds to nearest-even in the mantissa (no conversion unit).
 __device__ __forceinline__ uint32_t axis_fixed(float f) {
-    const float t = __fadd_rn(__fmul_rn(f, kAxisScale), 12582912.0f);
-    return __float_as_uint(t) - 0x4B400000u;
+    return __float_as_uint(__fmaf_rn(f, kAxisScale, kFloorMagic)) - kFloorMagicBits;
 }
 
-// Kinetic energy in eV (0.5 v^2/|q/m|, src/interpolation.cpp:88-89), clamped.
-__device__ __forceinline__ float energy_ev(float vx, float vy, float vz, float half_inv_abs_qm) {
+// Kinetic energy (0.5 v^2/|q/m|, src/interpolation.cpp:88-89) in units of
+// 2^-22 eV, clamped below 1024 eV; escale = escale * 2^22 (a power
+// of two: the product rounds as the energy in eV would).
+__device__ __forceinline__ float energy_units(float vx, float vy, float vz, float escale) {
     const float v2 = __fmaf_rn(vz, vz, __fmaf_rn(vy, vy, __fmul_rn(vx, vx)));
-    return fminf(__fmul_rn(v2, half_inv_abs_qm), kEnergyClampEv);
+    return fminf(__fmul_rn(v2, escale), kEnergyClampEv * kEnergyScale);
 }
 
 // Energy-weighted corner weights of one particle, rounded to integers of
@@ -248,8 +281,7 @@ struct EWeights {
     uint32_t e00, e10, e01, e11;
 };
 
-__device__ __forceinline__ EWeights energy_weights(float fx, float fy, float en) {
-    const float es = __fmul_rn(en, kEnergyScale);
+__device__ __forceinline__ EWeights energy_weights(float fx, float fy, float es) {
     const float a = __fmul_rn(es, __fsub_rn(1.0f, fx)), b = __fmul_rn(es, fx);
     const float ofy = __fsub_rn(1.0f, fy);
     EWeights w;
@@ -271,7 +303,7 @@ __device__ __forceinline__ void red_add(unsigned long long* p, unsigned long lon
 // weights (they sum to exactly 2^40).
 template <bool ENERGY>
 __device__ __forceinline__ void deposit_one(unsigned long long* acc_q, unsigned long long* acc_e,
-                                            int GX, uint32_t n, float fx, float fy, float en) {
+                                            int GX, uint32_t n, float fx, float fy, float es) {
     const uint32_t ax = axis_fixed(fx), ay = axis_fixed(fy);
     const uint32_t bx = kAxisOne - ax, by = kAxisOne - ay;
     red_add(acc_q + n, (unsigned long long)bx * by);
@@ -279,7 +311,7 @@ __device__ __forceinline__ void deposit_one(unsigned long long* acc_q, unsigned 
     red_add(acc_q + n + GX, (unsigned long long)bx * ay);
     red_add(acc_q + n + GX + 1, (unsigned long long)ax * ay);
     if (ENERGY) {
-        const EWeights e = energy_weights(fx, fy, en);
+        const EWeights e = energy_weights(fx, fy, es);
         red_add(acc_e + n, e.e00);
         red_add(acc_e + n + 1, e.e10);
         red_add(acc_e + n + GX, e.e01);
@@ -287,80 +319,101 @@ __device__ __forceinline__ void deposit_one(unsigned long long* acc_q, unsigned 
     }
 }
 
-// Per-lane sums of the particles that stay in the warp's cell.  Charge as
-// moments of the 20-bit axis weights -- count N (the warp's stayer count,
-// kept by the caller), sum ax, sum ay, sum ax*ay -- from which the four
-// corner sums follow exactly:
+// Per-lane sums of the particles that stay in the lane's cell.  Charge as
+// moments of the 20-bit axis weights -- sum ax, sum ay, sum ax*ay, and the
+// cell's stayer count N (kept by the caller) -- from which the four corner
+// sums follow exactly:
 //   Q00 = N 2^40 - (SX + SY) 2^20 + SXY,  Q10 = SX 2^20 - SXY,
 //   Q01 = SY 2^20 - SXY,                   Q11 = SXY.
-// A lane holds at most kMaxPerCell/32 = 2^11 particles: SX, SY < 2^31,
-// SXY < 2^51.  The energy mesh (a diagnostic) sums its corner weights per
-// lane in FP32, in 2^-22 eV units (< 2^43), rounded to integers once per
-// lane and cell: exact integer sums from there on, but the per-lane FP32
-// rounding depends on the order of the lane's particles.
+// A lane adds at most kFlushChunks = 2^11 particles between flushes: SX, SY
+// < 2^32, SXY < 2^52.  The energy mesh (a diagnostic) sums its corner weights
+// as integers of 2^-22 eV (each below 2^32, rounded once per particle).
+// Every sum is one of integers: no result depends on the order.
+constexpr uint32_t kFlushChunks = 1u << 11;
+
 struct StayAcc {
     uint32_t sx, sy;
     unsigned long long sxy;
-    float e[4];
+    unsigned long long e[4];
 };
 
 __device__ __forceinline__ void acc_zero(StayAcc& s) {
     s.sx = s.sy = 0u;
     s.sxy = 0ull;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) s.e[k] = 0.f;
+    for (int k = 0; k < 4; ++k) s.e[k] = 0ull;
 }
 
+// es: the particle's energy in units of 2^-22 eV
 template <bool ENERGY>
-__device__ __forceinline__ void acc_add(StayAcc& s, float fx, float fy, float en) {
+__device__ __forceinline__ void acc_add(StayAcc& s, float fx, float fy, float es) {
     const uint32_t ax = axis_fixed(fx), ay = axis_fixed(fy);
     s.sx += ax;
     s.sy += ay;
     s.sxy += (unsigned long long)ax * ay;
     if (ENERGY) {
-        const float es = __fmul_rn(en, kEnergyScale);
-        const float a = __fmul_rn(es, __fsub_rn(1.0f, fx)), b = __fmul_rn(es, fx);
-        const float ofy = __fsub_rn(1.0f, fy);
-        s.e[0] = __fmaf_rn(a, ofy, s.e[0]);
-        s.e[1] = __fmaf_rn(b, ofy, s.e[1]);
-        s.e[2] = __fmaf_rn(a, fy, s.e[2]);
-        s.e[3] = __fmaf_rn(b, fy, s.e[3]);
+        const EWeights w = energy_weights(fx, fy, es);
+        s.e[0] += w.e00;
+        s.e[1] += w.e10;
+        s.e[2] += w.e01;
+        s.e[3] += w.e11;
     }
 }
 
-// Warp sum of a value below 2^(LO+27) as two 32-bit limbs (redux.sync).
-template <int LO>
-__device__ __forceinline__ unsigned long long warp_sum_limbs(unsigned long long v) {
-    const uint32_t lo = (uint32_t)(v & ((1ull << LO) - 1ull));
-    const uint32_t hi = (uint32_t)(v >> LO);
-    return (unsigned long long)__reduce_add_sync(kFull, lo) +
-           ((unsigned long long)__reduce_add_sync(kFull, hi) << LO);
+// Sums v[0..NV) over the G lanes of a group (gl: the lane's index in it) by
+// recursive halving: a step exchanges half of the values still held, so the
+// whole reduction is NV - 1 exchanges (not NV log2 G) and ends with lane gl
+// holding the NV / G (at least one) totals from index `idx` on.  With G > NV
+// the G / NV lanes of equal idx hold the same total.
+template <int G, int NV>
+__device__ __forceinline__ int group_reduce_scatter(unsigned long long (&v)[NV], int gl) {
+    int idx = 0, cnt = NV;
+#pragma unroll
+    for (int d = G / 2; d >= 1; d >>= 1) {
+        if (cnt > 1) {
+            cnt >>= 1;
+            const bool hi = (gl & d) != 0;
+#pragma unroll
+            for (int k = 0; k < NV / 2; ++k)
+                if (k < cnt) {
+                    const unsigned long long send = hi ? v[k] : v[k + cnt];
+                    const unsigned long long keep = hi ? v[k + cnt] : v[k];
+                    v[k] = keep + __shfl_xor_sync(kFull, send, d);
+                }
+            idx += hi ? cnt : 0;
+        } else {
+            v[0] += __shfl_xor_sync(kFull, v[0], d);
+        }
+    }
+    return idx;
 }
 
-// Warp-reduce the cell's stayer sums and add them to its four nodes (lane 0).
-// N: the cell's stayer count (known to the whole warp).
-template <bool ENERGY>
-__device__ __forceinline__ void acc_flush(StayAcc& s, const KArgs& A, int gx, int gy, int lane,
-                                          unsigned long long N) {
-    const unsigned long long SX = warp_sum_limbs<26>(s.sx);
-    const unsigned long long SY = warp_sum_limbs<26>(s.sy);
-    const unsigned long long SXY = warp_sum_limbs<26>(s.sxy);
-    unsigned long long E[4] = {0ull, 0ull, 0ull, 0ull};
+// Reduces the stayer sums over each cell's group of G lanes and adds them to
+// the cell's four nodes (n0: its lower left node), one RED per lane for
+// G = 8: lane gl of the group holds quantity gl (charge corners 00, 10, 01,
+// 11, then the energy's).  N: the cell's stayer count.
+template <int G, bool ENERGY>
+__device__ __forceinline__ void acc_flush(StayAcc& s, const KArgs& A, uint32_t n0, int gl, uint32_t N) {
+    constexpr int NV = ENERGY ? 8 : 4;
+    unsigned long long v[NV];
+    const unsigned long long sx = (unsigned long long)s.sx << kAxisBits, sy = (unsigned long long)s.sy << kAxisBits;
+    v[3] = s.sxy;
+    v[2] = sy - s.sxy;
+    v[1] = sx - s.sxy;
+    v[0] = s.sxy - sx - sy;
     if (ENERGY) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) E[k] = warp_sum_limbs<22>(__float2ull_rn(s.e[k]));
+        for (int k = 0; k < 4; ++k) v[NV - 4 + k] = s.e[k];
     }
-    if (lane == 0 && N) {
-        const int64_t n = (int64_t)gy * A.GX + gx;
-        red_add(A.acc_q + n, (N << 40) - ((SX + SY) << 20) + SXY);
-        red_add(A.acc_q + n + 1, (SX << 20) - SXY);
-        red_add(A.acc_q + n + A.GX, (SY << 20) - SXY);
-        red_add(A.acc_q + n + A.GX + 1, SXY);
-        if (ENERGY) {
-            red_add(A.acc_e + n, E[0]);
-            red_add(A.acc_e + n + 1, E[1]);
-            red_add(A.acc_e + n + A.GX, E[2]);
-            red_add(A.acc_e + n + A.GX + 1, E[3]);
+    const int idx0 = group_reduce_scatter<G, NV>(v, gl);
+    constexpr int kPer = NV > G ? NV / G : 1, kSame = G > NV ? G / NV : 1;
+    if (N && (gl & (kSame - 1)) == 0) {
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int idx = idx0 + k;
+            unsigned long long* acc = (ENERGY && idx >= 4) ? A.acc_e : A.acc_q;
+            const uint32_t node = n0 + (idx & 1) + ((idx & 2) ? (uint32_t)A.GX : 0u);
+            red_add(acc + node, idx == 0 ? v[k] + ((unsigned long long)N << (2 * kAxisBits)) : v[k]);
         }
     }
     acc_zero(s);
@@ -368,8 +421,8 @@ __device__ __forceinline__ void acc_flush(StayAcc& s, const KArgs& A, int gx, in
 
 __device__ __forceinline__ void store_slot(float4* dst_a, float* dst_vz, uint32_t slot,
                                            const Pushed& p, float vz) {
-    __stcs(dst_a + slot, make_float4(p.fx, p.fy, p.vx, p.vy));
-    __stcs(dst_vz + slot, vz);
+    dst_a[slot] = make_float4(p.fx, p.fy, p.vx, p.vy);
+    dst_vz[slot] = vz;
 }
 
 // Appends the lanes with `on` set to a side list (one atomic per warp).
@@ -394,358 +447,321 @@ __device__ __forceinline__ void list_append(const ListDev& L, bool on, uint32_t 
     }
 }
 
-// One kernel body for the two uses:
+// One kernel body for three uses:
 //   kPush    -- push, place every particle in the other buffer, deposit the
-//               new positions;
-//   kDeposit -- deposit the current positions (no push, nothing moves).
-// A block owns a kTileX x kTileY tile of cells.  Its prologue stages the
-// tile's per-cell slot metadata and the node fields in shared memory; then
-// each warp streams through the particles of its cells (tile cells warp,
-// warp + kWarps, ...) in chunks of 32.  The chunks travel through a per-warp
-// ring of kDepth chunk buffers in shared memory filled by cp.async, kDepth-1
-// chunks ahead of the one being processed -- across cell boundaries, so the
-// load pipeline never drains.
-constexpr int kDepth = 4;
-static_assert((kDepth & (kDepth - 1)) == 0, "ring depth: a power of two");
+//               new positions of those that kept their cell;
+//   kDeposit -- deposit the current positions (no push, nothing moves);
+//   kArrivals -- deposit the back runs alone: what a push placed there.
+// A block owns a tile of TX x TY cells (powers of two, at most kTileCells).
+// Its prologue stages the tile's per-cell slot metadata and the node fields
+// in shared memory; then each warp works on sets of 32 / G neighbouring cells
+// of a row at a time, G lanes a cell: a chunk is the next 2 G particles of
+// each of the set's cells, two a lane.  The chunks travel through a per-warp
+// ring of kDepth chunk buffers in shared memory filled by cp.async, kDepth - 1
+// chunks ahead of the one being worked on -- across sets, so the load
+// pipeline never drains.
+constexpr int kTileCells = 256;  // (a queued particle's old cell is 8 bits)
+constexpr int kTileNodes = 2 * (kTileCells + 1);  // of the widest tile, 256 x 1 (the most nodes)
+
+// Blocks of 4 warps, 6 an SM (80 registers a thread): with 8 warps and a ring
+// of 2, and with 8 blocks of 4 warps at 64 registers, the push of the 1024^2
+// workload took 3 to 8 % longer.
+constexpr int kCellBlocksPerSM = 6;
+constexpr int kDepth = 3;  // chunks in the ring  // chunks in the ring
+
+struct Tile {
+    int ltx, lty;  // log2 of the cells in x and y
+};
 
 struct CellMeta {
     uint32_t b0, b1, nf, nb;
 };
 
-// Movers wait in a per-warp queue in shared memory and are placed 32 at a
-// time (all lanes busy): deposit, grouping by target cell (match.any), one
-// slot reservation per group, store.
-constexpr int kQueue = 64;
+// Particles that left their cell wait in a per-warp queue in shared memory
+// and are placed 32 at a time (all lanes busy): cell bookkeeping, deposit,
+// grouping by target cell (match.any), one slot reservation per group, store.
+constexpr int kQueue = 96;  // 31 waiting and a chunk of 64
 
 struct MoverQueue {
-    float4 a[kQueue];
+    float4 a[kQueue];  // position in units of the old cell (its corner at 0), vx, vy
     float vz[kQueue];
-    uint2 g[kQueue];  // target cell (gx, gy)
+    uint8_t cell[kQueue];  // old cell (index in the tile)
 };
 
-// A cell strictly inside its block's tile (not on the tile's border, not on
-// the periodic seam) receives direct placements only from cells of the
-// same tile: one-cell movers from elsewhere cannot reach it, and longer
-// jumps into it from other tiles go to the side list.  Its back count is
-// kept in shared memory and written out when the block ends, instead of a
-// global atomic per group of movers.  (lx, ly): the cell's position in its
-// tile; gy: its row.
-template <int TX, int TY>
-__device__ __forceinline__ bool tile_owned(int lx, int ly, int gy, const KArgs& A) {
-    return TY > 2 && lx >= 1 && lx <= TX - 2 && ly >= 1 && ly <= TY - 2 &&
-           !(A.k.pery && (gy == 0 || gy == A.ny - 1));
-}
-
-// Places `count` (<= 32) queued movers, entries 0..count-1, from the block
-// of tile (tgx0, tgy0): all lanes busy on the target's bookkeeping.
-template <bool ENERGY, int TX, int TY>
-__device__ __forceinline__ void place_movers(const KArgs& A, MoverQueue& q,
-                                             const CellMeta* __restrict__ s_meta,
-                                             uint32_t* s_back, int tgx0, int tgy0, int count,
-                                             int lane, unsigned lt) {
+// Places `count` (<= 32) queued particles from entry `first` on, of the block
+// with tile origin (tgx0, tgy0), one a lane: each reserves a slot at the back
+// of its new cell with one atomic, capped at the cell's capacity minus its
+// current count (the most stayers it can have).  Their deposit is left to
+// the pass over the arrivals (kArrivals).  Returns 1 in lanes whose particle
+// left through x < 0.
+__device__ __forceinline__ uint32_t place_movers(const KArgs& A, MoverQueue& q,
+                                                 const CellMeta* __restrict__ s_meta, Tile T, int tgx0,
+                                                 int tgy0, int first, int count, int lane, unsigned lt) {
     __syncwarp();
-    const bool on = lane < count;
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    Pushed p{};
     float vz = 0.f;
-    uint2 g = make_uint2(0u, 0u);
-    if (on) {
-        a = q.a[lane];
-        vz = q.vz[lane];
-        g = q.g[lane];
-    }
-    const uint32_t t = g.y * (uint32_t)A.nx + g.x;
-    const float en = (ENERGY && on) ? energy_ev(a.z, a.w, vz, A.k.half_inv_abs_qm) : 0.f;
-    // movers bound for the same cell form a group; its leader reserves the
-    // group's slots at the back of the cell, capped at the cell's capacity
-    // minus its current count (the most stayers it can have)
-    const unsigned grp = __match_any_sync(kFull, on ? t : (0x80000000u | (uint32_t)lane));
-    const int leader = __ffs(grp) - 1;
-    uint32_t old = 0, lim = 0, top = 0;
-    if (on && lane == leader) {
-        const uint32_t cnt = __popc(grp);
-        const int lx = (int)g.x - tgx0, ly = (int)g.y - tgy0;
-        const bool in_tile = (unsigned)lx < (unsigned)TX && (unsigned)ly < (unsigned)TY;
-        // the target's slots and source counts: from the tile's shared
-        // metadata when it lies in this block's tile (most movers go one
-        // cell), else from global memory
-        CellMeta m;
-        if (in_tile) {
-            m = s_meta[ly * TX + lx];
-        } else {
-            m.b0 = A.base[t];
-            m.b1 = A.base[t + 1];
-            m.nf = A.front_src[t];
-            m.nb = A.back_src[t];
-        }
-        lim = (m.b1 - m.b0) - (m.nf + m.nb);
-        top = m.b1;
-        // the back count: in shared memory for a cell this block owns
-        uint32_t* ctr = (in_tile && tile_owned<TX, TY>(lx, ly, (int)g.y, A)) ? s_back + (ly * TX + lx)
-                                                                              : A.back_dst + t;
-        old = atomicAdd(ctr, cnt);
-        // give back what does not fit (the count then ends at
-        // min(requested, lim) with slots 0.. taken)
-        if (old + cnt > lim) atomicSub(ctr, old >= lim ? cnt : old + cnt - lim);
-    }
-    if (on) deposit_one<ENERGY>(A.acc_q, A.acc_e, A.GX, g.y * (uint32_t)A.GX + g.x, a.x, a.y, en);
-    old = __shfl_sync(kFull, old, leader);
-    lim = __shfl_sync(kFull, lim, leader);
-    top = __shfl_sync(kFull, top, leader);
+    uint32_t left = 0, t = 0;
     bool spill = false;
-    Pushed p;
-    p.fx = a.x; p.fy = a.y; p.vx = a.z; p.vy = a.w;
-    if (on) {
-        const uint32_t k = old + __popc(grp & lt);
-        if (k < lim) store_slot(A.dst_a, A.dst_vz, top - 1u - k, p, vz);
-        else spill = true;
+    if (lane < count) {
+        const float4 a = q.a[first + lane];
+        const int lc = q.cell[first + lane];
+        vz = q.vz[first + lane];
+        p.px = a.x;
+        p.py = a.y;
+        p.vx = a.z;
+        p.vy = a.w;
+        recell(p);
+        resolve_move(p, A.k, tgx0 + (lc & ((1 << T.ltx) - 1)), tgy0 + (lc >> T.ltx), A.nx, A.ny);
+        if (p.alive) {
+            t = (uint32_t)p.gy * (uint32_t)A.nx + (uint32_t)p.gx;
+            const uint32_t k = atomicAdd(A.back_dst + t, 1u);
+            // the target's slots and source counts: from the tile's shared
+            // metadata when it lies in this block's tile, else from global
+            // memory
+            const int lx = p.gx - tgx0, ly = p.gy - tgy0;
+            CellMeta m;
+            if (((unsigned)lx >> T.ltx) == 0u && ((unsigned)ly >> T.lty) == 0u) {
+                m = s_meta[(ly << T.ltx) + lx];
+            } else {
+                m.b0 = A.base[t];
+                m.b1 = A.base[t + 1];
+                m.nf = A.front_src[t];
+                m.nb = A.back_src[t];
+            }
+            if (k < (m.b1 - m.b0) - (m.nf + m.nb)) {
+                store_slot(A.dst_a, A.dst_vz, m.b1 - 1u - k, p, vz);
+            } else {  // full: give the slot number back
+                atomicSub(A.back_dst + t, 1u);
+                spill = true;
+            }
+        } else {
+            left = p.left ? 1u : 0u;
+        }
     }
     list_append(A.ovf, spill, t, p, vz, lt, lane, A.counters + 2);
+    __syncwarp();
+    return left;
 }
 
-template <int MODE, bool ENERGY, int TX, int TY>
-__device__ __forceinline__ void cells_body(const KArgs& A, int tile_x, int tile_y) {
-    constexpr int kTileX = TX, kTileY = TY;
-    constexpr int kTileCells = kTileX * kTileY;
-    constexpr int kTileNodesX = kTileX + 1;
-    constexpr int kTileNodes = (kTileX + 1) * (kTileY + 1);
+template <int MODE, bool ENERGY, bool BZU, int G>
+__device__ __forceinline__ void cells_body(const KArgs& A, Tile T, uint32_t tile) {
+    constexpr int kSetCells = 32 / G;  // cells a warp works on at a time (neighbours in a row)
     __shared__ CellMeta s_meta[kTileCells];
-    __shared__ float4 s_fld[MODE == kPush ? kTileNodes : 1];
+    using Field = NodeField<BZU>;
+    __shared__ Field s_fld[MODE == kPush ? kTileNodes : 1];
     __shared__ MoverQueue s_q[MODE == kPush ? kWarps : 1];
-    // tiles of one or two rows own no cell
-    __shared__ uint32_t s_back[MODE == kPush && kTileY > 2 ? kTileCells : 1];
-    __shared__ float4 s_ring_a[kWarps][kDepth][32];
-    __shared__ float s_ring_vz[kWarps][kDepth][32];
+    __shared__ float4 s_ring_a[kWarps][kDepth][2][32];
+    __shared__ float s_ring_vz[kWarps][kDepth][2][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int tgx0 = tile_x * kTileX, tgy0 = tile_y * kTileY;
+    const int gl = lane & (G - 1), grp = lane / G;  // lane of the group, group of the warp
+    const int cells = 1 << (T.ltx + T.lty), sets = cells / kSetCells;
+    // tiles in row order: the blocks resident at a time work on one stretch
+    // of the slot arrays
+    const uint32_t tiles_x = (uint32_t)(A.nx + (1 << T.ltx) - 1) >> T.ltx, tile_y = tile / tiles_x;
+    const int tgx0 = (int)(tile - tile_y * tiles_x) << T.ltx, tgy0 = (int)tile_y << T.lty;
     const unsigned lt = lanemask_lt();
-    // tile cell (lx, ly) is owned: inside the grid, off the tile's border
-    // and off the periodic seam (rows 0 and ny-1 exchange wrapped movers)
-    auto owned = [&](int lx, int ly) {
-        return tgx0 + lx < A.nx && tgy0 + ly < A.ny && tile_owned<TX, TY>(lx, ly, tgy0 + ly, A);
-    };
-    if (MODE == kPush && kTileY > 2)
-        for (int i = threadIdx.x; i < kTileCells; i += kThreads) s_back[i] = 0u;
-    for (int i = threadIdx.x; i < kTileCells; i += kThreads) {
-        const int gx = tgx0 + (i % kTileX), gy = tgy0 + (i / kTileX);
+    const unsigned gmask = (G == 32 ? kFull : ((1u << (G & 31)) - 1u)) << (grp * G);
+    for (int i = threadIdx.x; i < cells; i += kThreads) {
+        const int gx = tgx0 + (i & ((1 << T.ltx) - 1)), gy = tgy0 + (i >> T.ltx);
         CellMeta m{0u, 0u, 0u, 0u};
         if (gx < A.nx && gy < A.ny) {
             const int64_t c = (int64_t)gy * A.nx + gx;
             m.b0 = A.base[c];
             m.b1 = A.base[c + 1];
-            m.nf = A.front_src[c];
+            m.nf = MODE == kArrivals ? 0u : A.front_src[c];
             m.nb = A.back_src[c];
         }
         s_meta[i] = m;
     }
+    const int rowlen = (1 << T.ltx) + 1;
     if (MODE == kPush) {
-        for (int i = threadIdx.x; i < kTileNodes; i += kThreads) {
-            const int x = tgx0 + (i % kTileNodesX), y = tgy0 + (i / kTileNodesX);
-            s_fld[i] = (x < A.GX && y < A.ny + 1) ? __ldg(A.fld + (int64_t)y * A.GX + x)
-                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+        const int nodes = rowlen * ((1 << T.lty) + 1);
+        for (int i = threadIdx.x; i < nodes; i += kThreads) {
+            const int ly = i / rowlen, x = tgx0 + (i - ly * rowlen), y = tgy0 + ly;
+            s_fld[i] = Field::from((x < A.GX && y < A.ny + 1) ? __ldg(A.fld + (int64_t)y * A.GX + x)
+                                                              : make_float4(0.f, 0.f, 0.f, 0.f));
         }
     }
     __syncthreads();
 
     uint32_t left_exits = 0;  // per lane
-    // the warp's cells are lc = warp + kWarps*k; empty ones only get their
-    // front count written
-    auto next_cell = [&](int lc, bool mark_empty) {
-        for (; lc < kTileCells; lc += kWarps) {
-            const CellMeta m = s_meta[lc];
-            if (m.nf + m.nb) break;
-            const int gx = tgx0 + (lc % kTileX), gy = tgy0 + (lc / kTileX);
-            if (MODE == kPush && mark_empty && lane == 0 && gx < A.nx && gy < A.ny)
-                A.front_dst[(int64_t)gy * A.nx + gx] = 0u;
+    // The set being loaded: the group's cell as the source index of its j-th
+    // particle (the front run for j < pnf, then the back run, index pback +
+    // j), its particle count pn, and the fullest cell's count pmax.
+    int pset = warp;
+    uint32_t pfront = 0, pback = 0, pnf = 0, pn = 0, pmax = 0, pj = 0;
+    auto p_enter = [&]() {  // the next set with particles, from pset on
+        for (; pset < sets; pset += kWarps) {
+            const CellMeta m = s_meta[pset * kSetCells + grp];
+            pn = m.nf + m.nb;
+            pmax = __reduce_max_sync(kFull, pn);
+            if (pmax) {
+                pfront = m.b0;
+                pnf = m.nf;
+                pback = m.b1 - pn;
+                break;
+            }
         }
-        return lc;
+        pj = gl;
     };
-    // producer: issues the copies of the chunk (plc, pj0) into ring slot r
-    // and advances; every call commits one (possibly empty) copy group
-    // the producer's cell as the source index of its j-th particle: the
-    // front run for j < nf, then the back run (index back + j)
-    struct ProdCell {
-        uint32_t front, back, nf, n;
-    };
-    auto prod_cell = [&](int c) {
-        const CellMeta pm = c < kTileCells ? s_meta[c] : CellMeta{0u, 0u, 0u, 0u};
-        return ProdCell{pm.b0, pm.b1 - pm.nb - pm.nf, pm.nf, pm.nf + pm.nb};
-    };
-    int plc = next_cell(warp, false);
-    ProdCell pc = prod_cell(plc);
-    uint32_t pj0 = 0;
-    const uint32_t ring_a0 = smem_u32(&s_ring_a[warp][0][lane]);
-    const uint32_t ring_vz0 = smem_u32(&s_ring_vz[warp][0][lane]);
-    auto issue = [&](int r) {
-        if (plc < kTileCells) {
-            const uint32_t jj = pj0 + lane;
-            const bool v = jj < pc.n;
-            const uint32_t i = !v ? 0u : (jj < pc.nf ? pc.front : pc.back) + jj;
-            cp_async16(ring_a0 + (uint32_t)r * (32u * 16u), A.src_a + i, v);
-            cp_async4(ring_vz0 + (uint32_t)r * (32u * 4u), A.src_vz + i, v);
-            if (pj0 + 32 >= pc.n) {
-                plc = next_cell(plc + kWarps, false);
-                pc = prod_cell(plc);
-                pj0 = 0;
-            } else {
-                pj0 += 32;
+    const uint32_t ring_a0 = smem_u32(&s_ring_a[warp][0][0][lane]);
+    const uint32_t ring_vz0 = smem_u32(&s_ring_vz[warp][0][0][lane]);
+    // issues the copies of the next chunk into ring slot r; every call
+    // commits one (possibly empty) copy group
+    auto fetch = [&](uint32_t r) {
+        if (pset < sets) {
+#pragma unroll
+            for (uint32_t u = 0; u < 2; ++u) {
+                const uint32_t j = pj + u * G;
+                if (j < pn) {
+                    const uint32_t i = (j < pnf ? pfront : pback) + j;
+                    cp_async16(ring_a0 + r * 1024u + u * 512u, A.src_a + i);
+                    cp_async4(ring_vz0 + r * 256u + u * 128u, A.src_vz + i);
+                }
+            }
+            pj += 2 * G;
+            if (pj - gl >= pmax) {
+                pset += kWarps;
+                p_enter();
             }
         }
         cp_async_commit();
     };
+    p_enter();
 
     MoverQueue& q = s_q[MODE == kPush ? warp : 0];
     int queued = 0;  // warp-uniform
-    int lc = next_cell(warp, true);
-    if (lc < kTileCells) {
-#pragma unroll
-        for (int r = 0; r < kDepth - 1; ++r) issue(r);
-        // the consumer's cell: particle count, coordinates, its field
-        // corner in the shared tile, and the next free front slot
-        uint32_t n, front;
-        int gx, gy;
-        const float4* f;
-        auto enter = [&](int c) {
-            const CellMeta m = s_meta[c];
+    // the set being worked on: the group's cell (index lc in the tile), its
+    // particle count n, its corner in the shared fields, its lower left node
+    // and the next free front slot; nmax: the fullest cell's count
+    int set = warp, lc = 0;
+    uint32_t n = 0, nmax = 0, front = 0, front0 = 0, node = 0, cell = 0;
+    bool inside = false;
+    const Field* f = s_fld;
+    auto enter = [&]() {  // the next set with particles; empty ones only get their front counts written
+        for (; set < sets; set += kWarps) {
+            lc = set * kSetCells + grp;
+            const CellMeta m = s_meta[lc];
             n = m.nf + m.nb;
-            front = m.b0;
-            const int lx = c % kTileX, ly = c / kTileX;
-            gx = tgx0 + lx;
-            gy = tgy0 + ly;
-            f = s_fld + ly * kTileNodesX + lx;
-        };
-        enter(lc);
-        uint32_t j0 = 0, front0 = front;
-        int r = 0;
+            nmax = __reduce_max_sync(kFull, n);
+            const int lx = lc & ((1 << T.ltx) - 1), ly = lc >> T.ltx;
+            const int gx = tgx0 + lx, gy = tgy0 + ly;
+            inside = gx < A.nx && gy < A.ny;
+            cell = (uint32_t)gy * (uint32_t)A.nx + (uint32_t)gx;
+            node = (uint32_t)gy * (uint32_t)A.GX + (uint32_t)gx;
+            front = front0 = m.b0;
+            f = s_fld + ly * rowlen + lx;
+            if (nmax) break;
+            if (MODE == kPush && gl == 0 && inside) A.front_dst[cell] = 0u;
+        }
+    };
+    enter();
+    if (set < sets) {
         StayAcc acc;
         acc_zero(acc);
+        uint32_t r = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kDepth - 1u; ++k) fetch(k);
+        uint32_t j0 = 0, jstop = min(nmax, kFlushChunks * G), counted = 0;
         for (;;) {
-            const bool last = j0 + 32 >= n;
-            // the next chunk: same cell, or the warp's next non-empty cell
-            const int lcn = last ? next_cell(lc + kWarps, true) : lc;
-            // refill the slot freed by the previous chunk, then wait for this one
-            issue((r + kDepth - 1) & (kDepth - 1));
+            fetch(r == 0 ? kDepth - 1u : r - 1u);  // refill the slot freed by the previous chunk
             cp_async_wait<kDepth - 1>();
-            const float4 a = s_ring_a[warp][r][lane];
-            const float vz = s_ring_vz[warp][r][lane];
-            r = (r + 1) & (kDepth - 1);
-
-            const bool valid = j0 + lane < n;
-            Pushed p;
-            bool stay;
-            if (MODE == kDeposit) {
-                p.fx = a.x; p.fy = a.y; p.vx = a.z; p.vy = a.w;
-                stay = valid;
-            } else {
-                p = push_move(a, f[0], f[1], f[kTileNodesX], f[kTileNodesX + 1], A.k);
-                stay = valid && (p.sx | p.sy) == 0;
-            }
-            const float en = (ENERGY && stay) ? energy_ev(p.vx, p.vy, vz, A.k.half_inv_abs_qm) : 0.f;
-            if (stay) acc_add<ENERGY>(acc, p.fx, p.fy, en);
+            Pushed p[2];
+            float vz[2];
+            bool stay[2], other[2];
+            Field f00, f10, f01, f11;
             if (MODE == kPush) {
-                const unsigned sm = __ballot_sync(kFull, stay);
-                if (stay) store_slot(A.dst_a, A.dst_vz, front + __popc(sm & lt), p, vz);
-                front += __popc(sm);
-                // the cell bookkeeping of the rest (absorbed or moving), only
-                // in chunks that have any (most chunks of slow species do not)
-                const bool other = valid && !stay;
-                if (__any_sync(kFull, other)) {
-                    bool mv = false, far = false;
-                    if (other) {
-                        resolve_move(p, A.k, gx, gy, A.nx, A.ny);
-                        mv = p.dir >= 0;
-                        // a jump of more than one cell into a cell that
-                        // another block owns: deposited here, placed from
-                        // the side list after the pass (rare)
-                        if (kTileY > 2 && p.dir == kFar) {
-                            const int olx = p.gx % kTileX, oly = p.gy % kTileY;
-                            const bool mine = p.gx - olx == tgx0 && p.gy - oly == tgy0;
-                            far = !mine && tile_owned<TX, TY>(olx, oly, p.gy, A);
-                            mv = mv && !far;
-                        }
-                        left_exits += (p.dir < 0 && p.left) ? 1u : 0u;
-                    }
-                    if (kTileY > 2 && __any_sync(kFull, far)) {
-                        const uint32_t tc = (uint32_t)(p.gy * A.nx + p.gx);
-                        if (far) {
-                            const float ef = ENERGY ? energy_ev(p.vx, p.vy, vz, A.k.half_inv_abs_qm) : 0.f;
-                            deposit_one<ENERGY>(A.acc_q, A.acc_e, A.GX, (uint32_t)(p.gy * A.GX + p.gx),
-                                                p.fx, p.fy, ef);
-                        }
-                        list_append(A.ovf, far, tc, p, vz, lt, lane, A.counters + 2);
-                    }
-                    const unsigned mm = __ballot_sync(kFull, mv);
-                    if (mm) {  // warp-uniform: queue the movers
-                        if (mv) {
-                            const int e = queued + __popc(mm & lt);
-                            q.a[e] = make_float4(p.fx, p.fy, p.vx, p.vy);
-                            q.vz[e] = vz;
-                            q.g[e] = make_uint2((uint32_t)p.gx, (uint32_t)p.gy);
-                        }
-                        queued += __popc(mm);
-                        if (queued >= 32) {
-                            place_movers<ENERGY, TX, TY>(A, q, s_meta, s_back, tgx0, tgy0, 32, lane, lt);
-                            // the rest (< 32) moves to the front of the queue
-                            queued -= 32;
-                            __syncwarp();
-                            if (lane < queued) {
-                                q.a[lane] = q.a[32 + lane];
-                                q.vz[lane] = q.vz[32 + lane];
-                                q.g[lane] = q.g[32 + lane];
-                            }
-                            __syncwarp();
-                        }
-                    }
+                f00 = f[0];
+                f10 = f[1];
+                f01 = f[rowlen];
+                f11 = f[rowlen + 1];
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float4 a = s_ring_a[warp][r][u][lane];
+                vz[u] = s_ring_vz[warp][r][u][lane];
+                const bool valid = j0 + gl + u * G < n;
+                if (MODE != kPush) {
+                    p[u].fx = a.x; p[u].fy = a.y; p[u].vx = a.z; p[u].vy = a.w;
+                    stay[u] = valid;
+                } else {
+                    p[u] = push_move<BZU>(a, f00, f10, f01, f11, A.k);
+                    p[u].fx = p[u].px;
+                    p[u].fy = p[u].py;
+                    stay[u] = valid && keeps_cell(p[u].px) && keeps_cell(p[u].py);
+                    other[u] = valid && !stay[u];
                 }
             }
-            if (last) {
-                const uint32_t stayers = front - front0;
-                acc_flush<ENERGY>(acc, A, gx, gy, lane, MODE == kPush ? stayers : n);
-                if (MODE == kPush && lane == 0) A.front_dst[(int64_t)gy * A.nx + gx] = stayers;
-                if (lcn >= kTileCells) break;
-                enter(lcn);
-                front0 = front;
-                j0 = 0;
-            } else {
-                j0 += 32;
+            r = r == kDepth - 1u ? 0u : r + 1u;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                unsigned sm = 0;
+                if (MODE == kPush) sm = __ballot_sync(kFull, stay[u]) & gmask;
+                if (stay[u]) {
+                    const float es = ENERGY ? energy_units(p[u].vx, p[u].vy, vz[u], A.k.escale) : 0.f;
+                    acc_add<ENERGY>(acc, p[u].fx, p[u].fy, es);
+                    if (MODE == kPush) store_slot(A.dst_a, A.dst_vz, front + __popc(sm & lt), p[u], vz[u]);
+                }
+                if (MODE == kPush) front += __popc(sm);
             }
-            lc = lcn;
+            if (MODE == kPush && __any_sync(kFull, other[0] || other[1])) {
+                // the rest (moving or absorbed) is queued
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const unsigned om = __ballot_sync(kFull, other[u]);
+                    if (other[u]) {
+                        const int e = queued + __popc(om & lt);
+                        q.a[e] = make_float4(p[u].px, p[u].py, p[u].vx, p[u].vy);
+                        q.vz[e] = vz[u];
+                        q.cell[e] = (uint8_t)lc;
+                    }
+                    queued += __popc(om);
+                }
+                while (queued >= 32) {
+                    queued -= 32;  // the last 32 of the queue
+                    left_exits += place_movers(A, q, s_meta, T, tgx0, tgy0, queued, 32, lane, lt);
+                }
+            }
+            j0 += 2 * G;
+            if (j0 >= jstop) {  // the set is done (or the per-lane sums are full)
+                const uint32_t stayers = MODE == kPush ? front - front0 : min(n, j0);
+                acc_flush<G, ENERGY>(acc, A, node, gl, stayers - counted);
+                counted = stayers;
+                if (j0 >= nmax) {
+                    if (MODE == kPush && gl == 0 && inside) A.front_dst[cell] = stayers;
+                    set += kWarps;
+                    enter();
+                    if (set >= sets) break;
+                    j0 = 0;
+                    counted = 0;
+                }
+                jstop = min(nmax, j0 + kFlushChunks * G);
+            }
         }
-        cp_async_wait<0>();
     }
-    if (MODE == kPush && queued > 0)
-        place_movers<ENERGY, TX, TY>(A, q, s_meta, s_back, tgx0, tgy0, queued, lane, lt);
     if (MODE == kPush) {
+        if (queued > 0) left_exits += place_movers(A, q, s_meta, T, tgx0, tgy0, 0, queued, lane, lt);
         const uint32_t left = __reduce_add_sync(kFull, left_exits);
         if (lane == 0 && left) atomicAdd(A.counters, (unsigned long long)left);
-        // the owned cells' back counts (no other block placed into them)
-        if (kTileY > 2) {
-            __syncthreads();
-            for (int i = threadIdx.x; i < kTileCells; i += kThreads) {
-                const int lx = i % kTileX, ly = i / kTileX;
-                if (owned(lx, ly) && s_back[i])
-                    A.back_dst[(int64_t)(tgy0 + ly) * A.nx + tgx0 + lx] = s_back[i];
-            }
-        }
     }
 }
 
-// Tile shapes the kernels are built for (cells per block in x, y); every
-// shape has 256 cells.
-#define PIC_TILE_SHAPES(X) X(64, 4) X(256, 1) X(128, 2) X(16, 16)
+// The tiles of the tile shapes 1, 2 and 3 (256 cells), and the two that shape
+// 0 chooses from (auto_tile).
 constexpr int kNumTileShapes = 4;
-constexpr int kTileShapeX[kNumTileShapes] = {64, 256, 128, 16};
-constexpr int kTileShapeY[kNumTileShapes] = {4, 1, 2, 16};
+constexpr int kNumTiles = 5;
+constexpr Tile kTile[kNumTiles] = {{5, 0}, {8, 0}, {7, 1}, {4, 4}, {6, 0}};
 
-template <int MODE, bool ENERGY, int TX, int TY>
-__global__ void __launch_bounds__(kThreads, kCellBlocksPerSM) k_cells(KArgs A) {
-    cells_body<MODE, ENERGY, TX, TY>(A, blockIdx.x, blockIdx.y);
+template <int MODE, bool ENERGY, bool BZU, int G>
+__global__ void __launch_bounds__(kThreads, kCellBlocksPerSM) k_cells(KArgs A, Tile T) {
+    cells_body<MODE, ENERGY, BZU, G>(A, T, blockIdx.x);
 }
 
-// One launch over many instances: block b works on tile (work[b].y & 0xffff,
-// work[b].y >> 16) of instance work[b].x, whose arguments are args[work[b].x].
-template <int MODE, bool ENERGY, int TX, int TY>
+// One launch over many instances: block b works on tile work[b].y of instance
+// work[b].x, whose arguments are args[work[b].x].
+template <int MODE, bool ENERGY, bool BZU, int G>
 __global__ void __launch_bounds__(kThreads, kCellBlocksPerSM) k_cells_batch(const KArgs* __restrict__ args,
-                                                             const uint2* __restrict__ work) {
+                                                             const uint2* __restrict__ work, Tile T) {
     __shared__ KArgs s_args;
     const uint2 w = work[blockIdx.x];
     static_assert(sizeof(KArgs) % 8 == 0, "KArgs copy");
@@ -753,7 +769,7 @@ __global__ void __launch_bounds__(kThreads, kCellBlocksPerSM) k_cells_batch(cons
         reinterpret_cast<unsigned long long*>(&s_args)[i] =
             reinterpret_cast<const unsigned long long*>(args + w.x)[i];
     __syncthreads();
-    cells_body<MODE, ENERGY, TX, TY>(s_args, (int)(w.y & 0xffffu), (int)(w.y >> 16));
+    cells_body<MODE, ENERGY, BZU, G>(s_args, T, w.y);
 }
 
 // ---- side lists ---------------------------------------------------------------
@@ -794,12 +810,10 @@ __global__ void __launch_bounds__(256) k_fixup(FixArgs F) {
             vz = F.prev.vz[i];
             p = push_one(F.prev.a[i], F.fld[n0], F.fld[n0 + 1], F.fld[n0 + F.GX], F.fld[n0 + F.GX + 1],
                          F.k, gx, gy, F.nx, F.ny);
-            if (p.dir < 0) {
+            if (!p.alive) {
                 if (p.left) atomicAdd(F.counters, 1ull);
                 continue;
             }
-            const float en = ENERGY ? energy_ev(p.vx, p.vy, vz, F.k.half_inv_abs_qm) : 0.f;
-            deposit_one<ENERGY>(F.acc_q, F.acc_e, F.GX, (uint32_t)(p.gy * F.GX + p.gx), p.fx, p.fy, en);
             t = (uint32_t)(p.gy * F.nx + p.gx);
         } else {
             const uint32_t e = i - n_prev;
@@ -808,6 +822,8 @@ __global__ void __launch_bounds__(256) k_fixup(FixArgs F) {
             vz = F.ovf.vz[e];
             t = F.ovf.cell[e];
         }
+        const float es = ENERGY ? energy_units(p.vx, p.vy, vz, F.k.escale) : 0.f;
+        deposit_one<ENERGY>(F.acc_q, F.acc_e, F.GX, t + t / (uint32_t)F.nx, p.fx, p.fy, es);  // node = t + gy
         const uint32_t lim = (F.base[t + 1] - F.base[t]) - F.front[t];
         const uint32_t k = atomicAdd(F.back + t, 1u);
         if (k < lim) {
@@ -828,13 +844,13 @@ __global__ void __launch_bounds__(256) k_fixup(FixArgs F) {
 
 // Deposit of the particles on a side list (stand-alone deposit).
 template <bool ENERGY>
-__global__ void __launch_bounds__(256) k_list_deposit(ListDev L, int nx, int GX, float half_inv_abs_qm,
+__global__ void __launch_bounds__(256) k_list_deposit(ListDev L, int nx, int GX, float escale,
                                                       unsigned long long* acc_q, unsigned long long* acc_e) {
     const uint32_t n = min(*L.count, L.cap);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 a = L.a[i];
         const uint32_t c = L.cell[i];
-        const float en = ENERGY ? energy_ev(a.z, a.w, L.vz[i], half_inv_abs_qm) : 0.f;
+        const float en = ENERGY ? energy_units(a.z, a.w, L.vz[i], escale) : 0.f;
         deposit_one<ENERGY>(acc_q, acc_e, GX, c + c / (uint32_t)nx, a.x, a.y, en);  // node = c + gy
     }
 }
@@ -842,8 +858,12 @@ __global__ void __launch_bounds__(256) k_list_deposit(ListDev L, int nx, int GX,
 // ---- layouts: counts, exclusive scans ------------------------------------------
 //
 // Slot capacity of a cell holding n particles: n + n/2 + 16 (room for a
-// step's incoming movers and for the count to drift between re-layouts).
-__host__ __device__ __forceinline__ uint32_t cell_capacity(uint32_t n) { return n + n / 2u + 16u; }
+// step's incoming movers and for the count to drift between re-layouts),
+// rounded up to a multiple of 8 so that every cell's run starts on a 128-byte
+// line of the float4 array and a 32-byte sector of vz (unaligned runs took
+// the Ar+ push of the 1024^2 workload from 0.93 to 1.03 ms: more lines and
+// sectors an access).
+__host__ __device__ __forceinline__ uint32_t cell_capacity(uint32_t n) { return (n + n / 2u + 23u) & ~7u; }
 
 // cnt[c] = front[c] + back[c]
 __global__ void k_cell_counts(const uint32_t* front, const uint32_t* back, int64_t ncells, uint32_t* cnt) {
@@ -1231,49 +1251,84 @@ KArgs make_args(pic_ctx* c, Species& sp) {
     return A;
 }
 
-dim3 tile_grid(const pic_ctx* c, int shape) {
-    return dim3((unsigned)((c->nx + kTileShapeX[shape] - 1) / kTileShapeX[shape]),
-                (unsigned)((c->ny + kTileShapeY[shape] - 1) / kTileShapeY[shape]));
+unsigned num_tiles(const pic_ctx* c, Tile T) {
+    return ((unsigned)(c->nx + (1 << T.ltx) - 1) >> T.ltx) * ((unsigned)(c->ny + (1 << T.lty) - 1) >> T.lty);
 }
 
-// Launch of k_cells with the tile shape `shape` (index into kTileShape*).
+// The tile of a shape for a species (or batch) of `ppc` particles a cell on
+// grids that 64 x 1 tiles cut into `tiles64`.  Shape 0 takes short one-row
+// tiles: the blocks resident at a time then work on one short stretch of the
+// slot arrays, and the last wave is short.  64 cells when they are sparse (a
+// block's prologue is shared by more work: 64 instances of 32 particles a
+// cell 3.67 ms a push of both species, 3.85 with 32 cells) and still fill
+// the device twice over; 32 otherwise (the 1024^2 workload 1.99 ms, 64 cells
+// 2.06, 256 x 1 2.21, 128 x 2 2.41, 16 x 16 2.90).
+int pick_tile(int shape, double ppc, int64_t tiles64) {
+    if (shape != 0) return shape;
+    return ppc < 48.0 && tiles64 >= 2 * 6 * 148 ? 4 : 0;
+}
+
+// Lanes a cell of a push.  Few lanes: a warp's set has more cells, so the
+// per-set work (metadata, reduction, REDs) is shared by more of them and
+// sparse cells leave fewer lanes idle; many lanes: longer contiguous runs an
+// access.  Measured, electron + ion push of a 512^2 grid in us with 4 / 8 /
+// 16 lanes: 4 particles a cell 100 / 114 / 169, 8: 118 / 126 / 174, 16: 168 /
+// 162 / 189, 32: 254 / 230 / 240, 48: 355 / 313 / 309, 64: 430 / 374 / 366.
+int pick_lanes(double ppc) { return ppc >= 48.0 ? 16 : (ppc >= 12.0 ? 8 : 4); }
+
+// What a launch of the cell kernels needs to know besides its arguments.
+struct CellLaunch {
+    int tile;   // index into kTile
+    int lanes;  // lanes a cell of a push
+    bool bzu;   // uniform Bz (in every instance)
+};
+
+CellLaunch cell_launch(const pic_ctx* c, const Species& sp) {
+    return CellLaunch{pick_tile(c->tile_shape, sp.ppc, num_tiles(c, kTile[4])), pick_lanes(sp.ppc),
+                      c->bz_uniform};
+}
+
+// A tenth to a fifth of a cell's electrons arrive a step, few of its ions:
+// 4 lanes (with the push's 16, arrivals of the 512^2 workload took 43 us of
+// mostly idle lanes instead of 22).
+constexpr int kDepositLanes = 8, kArrivalLanes = 4;
+
+// f(lanes a cell, uniform Bz) with both as compile-time constants
+template <typename F>
+void with_lanes(const CellLaunch& L, F&& f) {
+    auto go = [&](auto g) {
+        if (L.bzu) f(g, std::true_type());
+        else f(g, std::false_type());
+    };
+    if (L.lanes == 16) go(std::integral_constant<int, 16>());
+    else if (L.lanes == 8) go(std::integral_constant<int, 8>());
+    else go(std::integral_constant<int, 4>());
+}
+
 template <int MODE, bool ENERGY>
-void launch_cells(int shape, dim3 grid, cudaStream_t st, const KArgs& A) {
-    switch (shape) {
-        case 1: k_cells<MODE, ENERGY, 256, 1><<<grid, kThreads, 0, st>>>(A); break;
-        case 2: k_cells<MODE, ENERGY, 128, 2><<<grid, kThreads, 0, st>>>(A); break;
-        case 3: k_cells<MODE, ENERGY, 16, 16><<<grid, kThreads, 0, st>>>(A); break;
-        default: k_cells<MODE, ENERGY, 64, 4><<<grid, kThreads, 0, st>>>(A); break;
+void launch_cells(const CellLaunch& L, const pic_ctx* c, const KArgs& A) {
+    const Tile T = kTile[L.tile];
+    if constexpr (MODE == kPush) {
+        with_lanes(L, [&](auto g, auto bzu) {
+            k_cells<MODE, ENERGY, decltype(bzu)::value, decltype(g)::value><<<num_tiles(c, T), kThreads, 0, c->stream>>>(A, T);
+        });
+    } else {
+        constexpr int G = MODE == kDeposit ? kDepositLanes : kArrivalLanes;
+        k_cells<MODE, ENERGY, true, G><<<num_tiles(c, T), kThreads, 0, c->stream>>>(A, T);
     }
 }
 
 template <int MODE, bool ENERGY>
-void launch_cells_batch(int shape, unsigned nblocks, cudaStream_t st, const KArgs* args,
-                        const uint2* work) {
-    switch (shape) {
-        case 1: k_cells_batch<MODE, ENERGY, 256, 1><<<nblocks, kThreads, 0, st>>>(args, work); break;
-        case 2: k_cells_batch<MODE, ENERGY, 128, 2><<<nblocks, kThreads, 0, st>>>(args, work); break;
-        case 3: k_cells_batch<MODE, ENERGY, 16, 16><<<nblocks, kThreads, 0, st>>>(args, work); break;
-        default: k_cells_batch<MODE, ENERGY, 64, 4><<<nblocks, kThreads, 0, st>>>(args, work); break;
+void launch_cells_batch(const CellLaunch& L, unsigned nblocks, cudaStream_t st, const KArgs* args, const uint2* work) {
+    const Tile T = kTile[L.tile];
+    if constexpr (MODE == kPush) {
+        with_lanes(L, [&](auto g, auto bzu) {
+            k_cells_batch<MODE, ENERGY, decltype(bzu)::value, decltype(g)::value><<<nblocks, kThreads, 0, st>>>(args, work, T);
+        });
+    } else {
+        constexpr int G = MODE == kDeposit ? kDepositLanes : kArrivalLanes;
+        k_cells_batch<MODE, ENERGY, true, G><<<nblocks, kThreads, 0, st>>>(args, work, T);
     }
-}
-
-template <typename K>
-cudaError_t max_shared(K k) {
-    return cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                cudaSharedmemCarveoutMaxShared);
-}
-
-// Four blocks of the particle kernels per SM need ~4 x 44 KB of shared memory.
-template <int MODE, bool ENERGY>
-cudaError_t carveouts() {
-    cudaError_t e = cudaSuccess;
-#define PIC_CARVE(TX, TY)                                                           \
-    if (e == cudaSuccess) e = max_shared(k_cells<MODE, ENERGY, TX, TY>);           \
-    if (e == cudaSuccess) e = max_shared(k_cells_batch<MODE, ENERGY, TX, TY>);
-    PIC_TILE_SHAPES(PIC_CARVE)
-#undef PIC_CARVE
-    return e;
 }
 
 int check_flags(pic_ctx* c, Species& sp, bool sync);
@@ -1324,7 +1379,7 @@ int species_setup(pic_ctx* c, int s) {
     sp.k.h = (float)(0.5 * sp.ctom * c->cfg.dt);
     sp.k.dtdx = (float)(c->cfg.dt / c->dx);
     sp.k.dtdy = (float)(c->cfg.dt / c->dy);
-    sp.k.half_inv_abs_qm = sp.ctom != 0 ? (float)(0.5 / std::fabs(sp.ctom)) : 0.f;
+    sp.k.escale = sp.ctom != 0 ? (float)(0.5 / std::fabs(sp.ctom)) * kEnergyScale : 0.f;
     const size_t nc = (size_t)c->ncells;
     PIC_CUDA(cudaMalloc(&sp.base, (nc + 1) * sizeof(uint32_t)));
     PIC_CUDA(cudaMalloc(&sp.base_next, (nc + 1) * sizeof(uint32_t)));
@@ -1357,10 +1412,6 @@ int species_setup(pic_ctx* c, int s) {
     PIC_TRY(scan_cells<true>(c, sp, sp.cnt, sp.base, &total));
     PIC_TRY(grow_store(c, s, total));
     PIC_TRY(grow_lists(c, s));
-    PIC_CUDA((carveouts<kPush, true>()));
-    PIC_CUDA((carveouts<kPush, false>()));
-    PIC_CUDA((carveouts<kDeposit, true>()));
-    PIC_CUDA((carveouts<kDeposit, false>()));
     sp.acc_fresh = true;  // zero particles: the zero accumulator is their deposit
     return PIC_OK;
 }
@@ -1464,6 +1515,11 @@ int check_flags(pic_ctx* c, Species& sp, bool sync) {
 
 }  // namespace
 
+// Particles a cell, on average, of a layout of `slots` slots (cell_capacity).
+static double mean_count(const pic_ctx* c, uint32_t slots) {
+    return std::max(0.0, ((double)slots / (double)c->ncells - 19.5) / 1.5);
+}
+
 // Rebuilds the layout from the current per-cell counts (cell runs plus the
 // side list): every cell gets cell_capacity(count) slots with its particles
 // at the front.  Synchronises.
@@ -1477,6 +1533,7 @@ static int relayout(pic_ctx* c, int s) {
     c->launches += 2;
     uint32_t total = 0;
     PIC_TRY(scan_cells<true>(c, sp, sp.cnt, sp.base_next, &total));
+    sp.ppc = mean_count(c, total);
     const int dst = src ^ 1;
     if ((int64_t)total > sp.capacity) {
         // grow: a fresh store, the old current buffer copied into its buffer
@@ -1560,6 +1617,7 @@ static int fresh_layout(pic_ctx* c, int s) {
     sp.lcur = 0;
     sp.flags_pending = false;
     sp.host_flags[0] = 0u;
+    sp.ppc = mean_count(c, total);
     if ((int64_t)total > sp.capacity) {
         PIC_CUDA(cudaStreamSynchronize(c->stream));
         cudaFree(sp.store);
@@ -1682,14 +1740,14 @@ int particles_deposit(pic_ctx* c, int s) {
     const bool energy = c->cfg.deposit_energy != 0;
     const ListDev L = list_dev(sp.loose[sp.lcur]);
     prof_begin(c, PIC_PHASE_DEPOSIT);
-    const int sh = c->tile_shape;
+    const CellLaunch cl = cell_launch(c, sp);
     if (energy) {
-        launch_cells<kDeposit, true>(sh, tile_grid(c, sh), c->stream, A);
-        k_list_deposit<true><<<kFixupBlocks, 256, 0, c->stream>>>(L, c->nx, c->GX, sp.k.half_inv_abs_qm,
+        launch_cells<kDeposit, true>(cl, c, A);
+        k_list_deposit<true><<<kFixupBlocks, 256, 0, c->stream>>>(L, c->nx, c->GX, sp.k.escale,
                                                                   sp.acc_q, sp.acc_e);
     } else {
-        launch_cells<kDeposit, false>(sh, tile_grid(c, sh), c->stream, A);
-        k_list_deposit<false><<<kFixupBlocks, 256, 0, c->stream>>>(L, c->nx, c->GX, sp.k.half_inv_abs_qm,
+        launch_cells<kDeposit, false>(cl, c, A);
+        k_list_deposit<false><<<kFixupBlocks, 256, 0, c->stream>>>(L, c->nx, c->GX, sp.k.escale,
                                                                    sp.acc_q, sp.acc_e);
     }
     prof_end(c, PIC_PHASE_DEPOSIT);
@@ -1727,8 +1785,7 @@ int particles_push(pic_ctx* c, int s) {
         prof_end(c, PIC_PHASE_RELAYOUT);
     }
     KArgs A = make_args(c, sp);
-    const int sh = c->tile_shape;
-    const dim3 g = tile_grid(c, sh);
+    const CellLaunch cl = cell_launch(c, sp);
     const bool energy = c->cfg.deposit_energy != 0;
     const int dst = sp.cur ^ 1;
     PIC_CUDA(cudaMemsetAsync(sp.back[dst], 0, (size_t)c->ncells * 4, c->stream));
@@ -1737,9 +1794,18 @@ int particles_push(pic_ctx* c, int s) {
     PIC_CUDA(cudaMemsetAsync(sp.acc_e, 0, (size_t)c->nodes * 8, c->stream));
     prof_begin(c, PIC_PHASE_PUSH);
     if (energy)
-        launch_cells<kPush, true>(sh, g, c->stream, A);
+        launch_cells<kPush, true>(cl, c, A);
     else
-        launch_cells<kPush, false>(sh, g, c->stream, A);
+        launch_cells<kPush, false>(cl, c, A);
+    // the deposit of the particles that changed cell, from the back runs
+    KArgs B = A;
+    B.src_a = A.dst_a;
+    B.src_vz = A.dst_vz;
+    B.back_src = A.back_dst;
+    if (energy)
+        launch_cells<kArrivals, true>(cl, c, B);
+    else
+        launch_cells<kArrivals, false>(cl, c, B);
     prof_end(c, PIC_PHASE_PUSH);
     PIC_CUDA(cudaGetLastError());
     FixArgs F{};
@@ -1818,12 +1884,14 @@ int particles_time_shapes(pic_ctx* c, int reps, double* ms) {
             for (int s = 0; s < ns; ++s) {
                 Species& sp = c->sp[s];
                 KArgs A = make_args(c, sp);
+                CellLaunch cl = cell_launch(c, sp);
+                cl.tile = pick_tile(sh, sp.ppc, num_tiles(c, kTile[4]));
                 cudaMemsetAsync(sp.back[sp.cur ^ 1], 0, (size_t)c->ncells * 4, c->stream);
                 cudaMemsetAsync(sp.list_counts + kOvf, 0, sizeof(uint32_t), c->stream);
                 if (energy)
-                    launch_cells<kPush, true>(sh, tile_grid(c, sh), c->stream, A);
+                    launch_cells<kPush, true>(cl, c, A);
                 else
-                    launch_cells<kPush, false>(sh, tile_grid(c, sh), c->stream, A);
+                    launch_cells<kPush, false>(cl, c, A);
             }
             cudaEventRecord(e1, c->stream);
             if (cudaEventSynchronize(e1) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
@@ -1909,12 +1977,10 @@ __global__ void __launch_bounds__(256) k_fixup_batch(const FixArgs* __restrict__
             vz = F.prev.vz[i];
             p = push_one(F.prev.a[i], F.fld[n0], F.fld[n0 + 1], F.fld[n0 + F.GX], F.fld[n0 + F.GX + 1],
                          F.k, gx, gy, F.nx, F.ny);
-            if (p.dir < 0) {
+            if (!p.alive) {
                 if (p.left) atomicAdd(F.counters, 1ull);
                 continue;
             }
-            const float en = ENERGY ? energy_ev(p.vx, p.vy, vz, F.k.half_inv_abs_qm) : 0.f;
-            deposit_one<ENERGY>(F.acc_q, F.acc_e, F.GX, (uint32_t)(p.gy * F.GX + p.gx), p.fx, p.fy, en);
             t = (uint32_t)(p.gy * F.nx + p.gx);
         } else {
             const uint32_t e = i - n_prev;
@@ -1923,6 +1989,8 @@ __global__ void __launch_bounds__(256) k_fixup_batch(const FixArgs* __restrict__
             vz = F.ovf.vz[e];
             t = F.ovf.cell[e];
         }
+        const float es = ENERGY ? energy_units(p.vx, p.vy, vz, F.k.escale) : 0.f;
+        deposit_one<ENERGY>(F.acc_q, F.acc_e, F.GX, t + t / (uint32_t)F.nx, p.fx, p.fy, es);  // node = t + gy
         const uint32_t lim = (F.base[t + 1] - F.base[t]) - F.front[t];
         const uint32_t k = atomicAdd(F.back + t, 1u);
         if (k < lim) {
@@ -1960,9 +2028,9 @@ __global__ void k_batch_flags(const FlagEntry* __restrict__ e, int n, unsigned l
 
 struct ParticleBatchImpl {
     int n = 0, ns = 0;
-    uint2* work[kNumTileShapes] = {};
-    unsigned nblocks[kNumTileShapes] = {};
-    KArgs* d_args = nullptr;      // [ns][n]
+    uint2* work[kNumTiles] = {};
+    unsigned nblocks[kNumTiles] = {};
+    KArgs* d_args = nullptr;      // [ns][n] pushes, then [ns][n] deposits of arrivals
     FixArgs* d_fix = nullptr;     // [ns][n]
     FlushEntry* d_flush = nullptr;  // [ns][n]
     ZeroEntry* d_zero = nullptr;  // [ns][3n] before each push, [ns][2n] after, [n] rho
@@ -1974,6 +2042,8 @@ struct ParticleBatchImpl {
     size_t table_bytes = 0;
     unsigned long long* h_flags = nullptr;
     int64_t max_nodes = 0;  // nodes of the largest instance
+    double ppc = 0;         // particles a cell, over all instances and species
+    bool bzu = true;        // every instance's Bz is uniform
 };
 
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -1984,12 +2054,11 @@ int batch_create(pic_ctx** cs, int n, ParticleBatchImpl** out) {
     B->n = n;
     B->ns = cs[0]->cfg.num_species;
     for (int i = 0; i < n; ++i) B->max_nodes = std::max<int64_t>(B->max_nodes, cs[i]->nodes);
-    for (int sh = 0; sh < kNumTileShapes; ++sh) {
+    for (int sh = 0; sh < kNumTiles; ++sh) {
         std::vector<uint2> w;
         for (int i = 0; i < n; ++i) {
-            const dim3 g = tile_grid(cs[i], sh);
-            for (unsigned y = 0; y < g.y; ++y)
-                for (unsigned x = 0; x < g.x; ++x) w.push_back(make_uint2((uint32_t)i, x | (y << 16)));
+            const unsigned tiles = num_tiles(cs[i], kTile[sh]);
+            for (unsigned t = 0; t < tiles; ++t) w.push_back(make_uint2((uint32_t)i, t));
         }
         B->nblocks[sh] = (unsigned)w.size();
         PIC_CUDA(cudaMalloc(&B->work[sh], w.size() * sizeof(uint2)));
@@ -2002,7 +2071,7 @@ int batch_create(pic_ctx** cs, int n, ParticleBatchImpl** out) {
         off += align256(bytes);
         return o;
     };
-    const size_t o_args = carve(sizeof(KArgs) * ns * n), o_fix = carve(sizeof(FixArgs) * ns * n);
+    const size_t o_args = carve(sizeof(KArgs) * 2 * ns * n), o_fix = carve(sizeof(FixArgs) * ns * n);
     const size_t o_flush = carve(sizeof(FlushEntry) * ns * n), o_zero = carve(sizeof(ZeroEntry) * (ns * 5 * n + n));
     const size_t o_flag = carve(sizeof(FlagEntry) * ns * n);
     B->table_bytes = off;
@@ -2045,7 +2114,7 @@ int batch_prepare(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st) {
                 B->h_flags[4 * ((size_t)s * n + i)] = 0;
             }
         }
-    const size_t o_args = 0, o_fix = align256(sizeof(KArgs) * ns * n);
+    const size_t o_args = 0, o_fix = align256(sizeof(KArgs) * 2 * ns * n);
     const size_t o_flush = o_fix + align256(sizeof(FixArgs) * ns * n);
     const size_t o_zero = o_flush + align256(sizeof(FlushEntry) * ns * n);
     const size_t o_flag = o_zero + align256(sizeof(ZeroEntry) * (ns * 5 * n + n));
@@ -2054,14 +2123,26 @@ int batch_prepare(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st) {
     FlushEntry* hl = reinterpret_cast<FlushEntry*>(B->h_tables + o_flush);
     ZeroEntry* hz = reinterpret_cast<ZeroEntry*>(B->h_tables + o_zero);
     FlagEntry* hg = reinterpret_cast<FlagEntry*>(B->h_tables + o_flag);
+    B->bzu = true;
+    double cells = 0, count = 0;
     for (int i = 0; i < n; ++i) {
         pic_ctx* c = cs[i];
+        B->bzu = B->bzu && c->bz_uniform;
+        for (int s = 0; s < ns; ++s) {
+            cells += (double)c->ncells;
+            count += (double)c->ncells * c->sp[s].ppc;
+        }
         hz[(size_t)ns * 5 * n + i] = ZeroEntry{reinterpret_cast<uint32_t*>(c->rho), (uint64_t)c->nodes * 2};
         for (int s = 0; s < ns; ++s) {
             Species& sp = c->sp[s];
             const size_t k = (size_t)s * n + i;
             const int dst = sp.cur ^ 1;
             ha[k] = make_args(c, sp);
+            KArgs& B2 = ha[(size_t)ns * n + k];
+            B2 = ha[k];
+            B2.src_a = B2.dst_a;
+            B2.src_vz = B2.dst_vz;
+            B2.back_src = B2.back_dst;
             FixArgs& F = hf[k];
             F = FixArgs{};
             F.nx = c->nx;
@@ -2095,8 +2176,20 @@ int batch_prepare(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st) {
             hg[k] = FlagEntry{sp.list_counts + kLoose0 + (sp.lcur ^ 1), sp.counters};
         }
     }
+    B->ppc = count / cells;
     PIC_CUDA(cudaMemcpyAsync(B->d_tables, B->h_tables, B->table_bytes, cudaMemcpyHostToDevice, st));
     return PIC_OK;
+}
+
+static CellLaunch batch_launch(const ParticleBatchImpl* B, int shape) {
+    return CellLaunch{pick_tile(shape, B->ppc, B->nblocks[4]), pick_lanes(B->ppc), B->bzu};
+}
+
+// The kernels that a push of the batch launches, as a number: a captured
+// step is good for as long as it does not change.
+int batch_kernels(const ParticleBatchImpl* B, int shape) {
+    const CellLaunch L = batch_launch(B, shape);
+    return (L.tile * 64 + L.lanes) * 2 + (L.bzu ? 1 : 0);
 }
 
 // zero rho of every instance; flush the accumulators of every species into
@@ -2114,12 +2207,17 @@ int batch_deposit(ParticleBatchImpl* B, cudaStream_t st) {
 // flags for the host (copied into B->h_flags on `st`).
 int batch_push(ParticleBatchImpl* B, int shape, bool energy, cudaStream_t st) {
     const int n = B->n, ns = B->ns;
+    const CellLaunch cl = batch_launch(B, shape);
     for (int s = 0; s < ns; ++s) {
         k_batch_zero<<<296, 256, 0, st>>>(B->d_zero + (size_t)s * 5 * n, 3 * n);
         if (energy)
-            launch_cells_batch<kPush, true>(shape, B->nblocks[shape], st, B->d_args + (size_t)s * n, B->work[shape]);
+            launch_cells_batch<kPush, true>(cl, B->nblocks[cl.tile], st, B->d_args + (size_t)s * n, B->work[cl.tile]);
         else
-            launch_cells_batch<kPush, false>(shape, B->nblocks[shape], st, B->d_args + (size_t)s * n, B->work[shape]);
+            launch_cells_batch<kPush, false>(cl, B->nblocks[cl.tile], st, B->d_args + (size_t)s * n, B->work[cl.tile]);
+        if (energy)
+            launch_cells_batch<kArrivals, true>(cl, B->nblocks[cl.tile], st, B->d_args + (size_t)(ns + s) * n, B->work[cl.tile]);
+        else
+            launch_cells_batch<kArrivals, false>(cl, B->nblocks[cl.tile], st, B->d_args + (size_t)(ns + s) * n, B->work[cl.tile]);
         if (energy)
             k_fixup_batch<true><<<n * kFixupBlocksPerInstance, 256, 0, st>>>(B->d_fix + (size_t)s * n);
         else
@@ -2167,6 +2265,7 @@ int batch_time_shapes(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st, int r
     PIC_CUDA(cudaEventCreate(&e1));
     int status = PIC_OK;
     for (int sh = 0; sh < kNumTileShapes && status == PIC_OK; ++sh) {
+        const CellLaunch cl = batch_launch(B, sh);
         float total = 0.f;
         for (int r = -1; r < reps; ++r) {
             cudaEventRecord(e0, st);
@@ -2174,9 +2273,9 @@ int batch_time_shapes(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st, int r
                 k_batch_zero<<<296, 256, 0, st>>>(B->d_zero + (size_t)s * 5 * n, 3 * n);
                 k_batch_zero<<<1, 256, 0, st>>>(B->d_zero + (size_t)s * 5 * n + 3 * n, n);  // ovf counts
                 if (energy)
-                    launch_cells_batch<kPush, true>(sh, B->nblocks[sh], st, B->d_args + (size_t)s * n, B->work[sh]);
+                    launch_cells_batch<kPush, true>(cl, B->nblocks[cl.tile], st, B->d_args + (size_t)s * n, B->work[cl.tile]);
                 else
-                    launch_cells_batch<kPush, false>(sh, B->nblocks[sh], st, B->d_args + (size_t)s * n, B->work[sh]);
+                    launch_cells_batch<kPush, false>(cl, B->nblocks[cl.tile], st, B->d_args + (size_t)s * n, B->work[cl.tile]);
             }
             cudaEventRecord(e1, st);
             if (cudaEventSynchronize(e1) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
@@ -2234,7 +2333,7 @@ struct SourceArgs {
     unsigned long long* i_acc_q;
     unsigned long long* i_acc_e;
     int deposit_e, deposit_i, energy;
-    float e_half_inv_abs_qm, i_half_inv_abs_qm;
+    float e_escale, i_escale;
     unsigned long long* e_counters;
     unsigned long long* i_counters;
     unsigned* accepted;  // pairs created
@@ -2264,7 +2363,7 @@ template <bool ENERGY>
 __device__ __forceinline__ void append_point(const SourceArgs& S, const ListDev& L, double x, double y,
                                              double vx, double vy, double vz, bool deposit,
                                              unsigned long long* acc_q, unsigned long long* acc_e,
-                                             float half_inv_abs_qm, unsigned long long* counters) {
+                                             float escale, unsigned long long* counters) {
     const double sx = x * (1.0 / S.dx), sy = y * (1.0 / S.dy);
     if (!(sx >= 0.0 && sy >= 0.0 && sx < (double)S.nx && sy < (double)S.ny)) return;
     const int gx = (int)sx, gy = (int)sy;
@@ -2278,7 +2377,7 @@ __device__ __forceinline__ void append_point(const SourceArgs& S, const ListDev&
     L.vz[s] = (float)vz;
     L.cell[s] = (uint32_t)(gy * S.nx + gx);
     if (deposit) {
-        const float en = ENERGY ? energy_ev((float)vx, (float)vy, (float)vz, half_inv_abs_qm) : 0.f;
+        const float en = ENERGY ? energy_units((float)vx, (float)vy, (float)vz, escale) : 0.f;
         deposit_one<ENERGY>(acc_q, acc_e, S.GX, (uint32_t)(gy * S.GX + gx), fx, fy, en);
     }
 }
@@ -2295,7 +2394,7 @@ __global__ void k_sources(SourceArgs S) {
             maxwell(S.ve, r0, r1, vx, vy, vz);
             const uint4 r2 = philox(make_uint4(k, S.call, 2u, 0x50u), S.key);
             append_point<ENERGY>(S, S.e_list, S.x_reinject, S.H * u01d(r2.x, r2.y), vx, vy, vz, S.deposit_e,
-                                 S.e_acc_q, S.e_acc_e, S.e_half_inv_abs_qm, S.e_counters);
+                                 S.e_acc_q, S.e_acc_e, S.e_escale, S.e_counters);
         } else {
             // generate_pairs (src/utils.cpp:517-566): one electron and one
             // ion at x = xm + asin(2u-1)(x22-x11)/pi, y uniform, kept inside (0, W)
@@ -2308,10 +2407,10 @@ __global__ void k_sources(SourceArgs S) {
             double vx, vy, vz;
             maxwell(S.ve, r0, r1, vx, vy, vz);
             append_point<ENERGY>(S, S.e_list, x, y, vx, vy, vz, S.deposit_e, S.e_acc_q, S.e_acc_e,
-                                 S.e_half_inv_abs_qm, S.e_counters);
+                                 S.e_escale, S.e_counters);
             maxwell(S.vi, r3, r4, vx, vy, vz);
             append_point<ENERGY>(S, S.i_list, x, y, vx, vy, vz, S.deposit_i, S.i_acc_q, S.i_acc_e,
-                                 S.i_half_inv_abs_qm, S.i_counters);
+                                 S.i_escale, S.i_counters);
             atomicAdd(S.accepted, 1u);
         }
     }
@@ -2381,8 +2480,8 @@ int particles_generate(pic_ctx* c, const pic_source_desc* d, int64_t* n_e, int64
     S.i_acc_e = I.acc_e;
     S.deposit_e = E.acc_fresh ? 1 : 0;
     S.deposit_i = I.acc_fresh ? 1 : 0;
-    S.e_half_inv_abs_qm = E.k.half_inv_abs_qm;
-    S.i_half_inv_abs_qm = I.k.half_inv_abs_qm;
+    S.e_escale = E.k.escale;
+    S.i_escale = I.k.escale;
     S.e_counters = E.counters;
     S.i_counters = I.counters;
     S.accepted = accepted;

@@ -54,12 +54,12 @@ constexpr uint32_t kMaxPerCell = 1u << 16;
 // ---------------------------------------------------------------------------
 // Particle kernel tiling
 // ---------------------------------------------------------------------------
-constexpr int kWarps = 8;   // 256 threads per block (a tile of 256 cells)
+constexpr int kWarps = 4;   // of a block of the cell kernels
 
 struct SpeciesConsts {
     float h;          // 0.5*(q/m)*dt
     float dtdx, dtdy; // dt/dx, dt/dy
-    float half_inv_abs_qm;  // 0.5/|q/m| -> kinetic energy in eV
+    float escale;     // 0.5/|q/m| * 2^22: v^2 -> kinetic energy in units of 2^-22 eV
     // uniform Bz (bzu != 0): the Boris rotation factors t = h*Bz and
     // s = 2t/(1+t^2), the same for every particle
     int bzu;
@@ -104,6 +104,7 @@ struct Species {
     double ctom = 0, weighing = 0;
     SpeciesConsts k{};
     int64_t capacity = 0;           // slots per buffer
+    double ppc = 0;                 // particles a cell when the layout was made
     float* store = nullptr;         // 2 buffers x 5 arrays x capacity floats
     ParticleSoA buf[2]{};
     int cur = 0;
@@ -270,6 +271,7 @@ int batch_create(pic_ctx** cs, int n, ParticleBatchImpl** out);
 void batch_destroy(ParticleBatchImpl* B);
 int batch_prepare(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st);
 int batch_deposit(ParticleBatchImpl* B, cudaStream_t st);
+int batch_kernels(const ParticleBatchImpl* B, int shape);
 int batch_push(ParticleBatchImpl* B, int shape, bool energy, cudaStream_t st);
 void batch_commit(pic_ctx** cs, int n);
 int batch_time_shapes(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st, int reps, bool energy,

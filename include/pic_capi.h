@@ -245,7 +245,7 @@ int pic_write_diagnostics(pic_ctx* ctx, const char* dir, int iteration, double s
 
 /* ---- instrumentation (no reference counterpart; the reference returns
  * host wall seconds per operator, src/sycl_pic_ctypes.cpp:127-236) ------- */
-#define PIC_PHASE_PUSH 0         /* the push pass: gather, Boris, binning, fused deposit */
+#define PIC_PHASE_PUSH 0         /* the push pass: gather, Boris, binning, deposit        */
 #define PIC_PHASE_FIXUP 1        /* side list: movers whose target cell was full      */
 #define PIC_PHASE_RELAYOUT 2     /* slot-layout rebuilds (rare)                        */
 #define PIC_PHASE_DEPOSIT 3      /* stand-alone deposit of current positions          */
@@ -279,8 +279,9 @@ int pic_debug_set_wait_limits(pic_ctx* ctx, int64_t barrier_polls, int64_t tenso
 int pic_debug_vcycle(pic_ctx* ctx, const float* rhs, float* out, int per_sweep);
 
 /* ---- tuning (no reference counterpart) -----------------------------------
- * The particle kernels are built for PIC_NUM_TILE_SHAPES tile shapes of 256
- * cells: 0 = 64x4 (default), 1 = 256x1, 2 = 128x2, 3 = 16x16. */
+ * The particle kernels run on PIC_NUM_TILE_SHAPES tile shapes: 0 = one row of
+ * 32 or 64 cells, whichever suits the grid and the particles a cell (default),
+ * 1 = 256x1, 2 = 128x2, 3 = 16x16. */
 #define PIC_NUM_TILE_SHAPES 4
 int pic_set_tile_shape(pic_ctx* ctx, int tile_shape);
 /* Times the push of the current particles with every tile shape (the
