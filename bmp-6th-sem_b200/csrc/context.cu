@@ -677,7 +677,7 @@ int pic_zero_rho(pic_ctx* c) {
 int pic_charge_deposition(pic_ctx* c, int s) {
     PIC_TRY(check_species(c, s));
     if (!c->sp[s].acc_fresh) PIC_TRY(particles_deposit(c, s));
-    return particles_flush_rho(c, s);
+    return particles_flush(c, s, 1, false);
 }
 
 int pic_poisson_solve(pic_ctx* c, int iteration) {
@@ -709,8 +709,9 @@ int pic_particle_phase(pic_ctx* c, int iteration) {
 
 int pic_step(pic_ctx* c, int iteration) {
     if (!c) return fail(PIC_ERR_ARG, "null context");
-    PIC_TRY(pic_zero_rho(c));
-    for (int s = 0; s < c->cfg.num_species; ++s) PIC_TRY(pic_charge_deposition(c, s));
+    for (int s = 0; s < c->cfg.num_species; ++s)
+        if (!c->sp[s].acc_fresh) PIC_TRY(particles_deposit(c, s));
+    PIC_TRY(particles_flush(c, 0, c->cfg.num_species, true));
     PIC_TRY(pic_poisson_solve(c, iteration));
     for (int s = 0; s < c->cfg.num_species; ++s) PIC_TRY(pic_move_particles(c, s, iteration));
     return PIC_OK;

@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "pic_capi.h"
@@ -31,6 +32,28 @@ int fail(int status, const std::string& msg);
         int s_ = (call);             \
         if (s_ != PIC_OK) return s_; \
     } while (0)
+
+// ---------------------------------------------------------------------------
+// Programmatic dependent launch: the grid starts launching while the one
+// before it in the stream drains; its threads wait for that grid's end (and
+// its writes) at pdl_wait, called before anything else is read or written.
+// ---------------------------------------------------------------------------
+template <typename... P, typename... A>
+void launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
 // Fixed-point deposit scales
@@ -94,6 +117,18 @@ struct LooseList {
     uint32_t cap = 0;
 };
 
+// What a push tells the host (k_fixup), one 8-byte word: the side list's
+// length (low half), two error flags and the push's number modulo 2^30.
+constexpr uint32_t kReportSeqMask = (1u << 30) - 1u;
+__host__ __device__ constexpr unsigned long long push_report(uint32_t loose, bool cell_limit, bool lost, uint32_t seq) {
+    return (unsigned long long)loose | (cell_limit ? 1ull << 32 : 0ull) | (lost ? 1ull << 33 : 0ull) |
+           ((unsigned long long)(seq & kReportSeqMask) << 34);
+}
+inline uint32_t report_loose(unsigned long long f) { return (uint32_t)f; }
+inline bool report_cell_limit(unsigned long long f) { return (f >> 32) & 1; }
+inline bool report_lost(unsigned long long f) { return (f >> 33) & 1; }
+inline uint32_t report_seq(unsigned long long f) { return (uint32_t)(f >> 34); }
+
 // Slot layout.  Cell c owns slots base[c] .. base[c+1] of each buffer; its
 // particles are the front run base[c] .. base[c]+front[c] (those that stayed
 // in the cell at the last push, or all of them after a re-layout) and the
@@ -118,15 +153,17 @@ struct Species {
     LooseList ovf;                  // push output: not yet placed
     LooseList loose[2];             // [lcur]: part of the state, not yet placed
     int lcur = 0;
-    uint32_t* host_flags = nullptr; // pinned: loose count + counters after the last push
-    cudaEvent_t flags_ev = nullptr;
+    unsigned long long* flags = nullptr;  // pinned: the last push's report
+    uint32_t loose_count = 0;       // side-list length in the last report read
+    uint32_t push_seq = 0;          // pushes so far
     bool flags_pending = false;
     unsigned long long* acc_q = nullptr;  // [nodes] fixed-point charge weights
-    unsigned long long* acc_e = nullptr;  // [nodes] fixed-point energy weights
+    unsigned long long* acc_e = nullptr;  // [nodes] fixed-point energy weights (same allocation, after acc_q)
     double* final_mesh = nullptr;   // [nodes]
     double* energy_mesh = nullptr;  // [nodes]
     unsigned long long* counters = nullptr;  // [0] left exits, [1] cell limit, [2] lost particles
     bool acc_fresh = false;         // acc_* hold the deposit of the current positions
+    bool acc_clear = false;         // acc_* are zero
 };
 
 // Multigrid level (FP32).
@@ -261,7 +298,8 @@ int particles_load_plasma(pic_ctx* c, int s, const pic_plasma_desc* d);
 // raw state into 6 consecutive arrays of n entries (int32 cell, 5 floats)
 int particles_export_state(pic_ctx* c, int s, void* dev, int64_t n);
 int particles_deposit(pic_ctx* c, int s);       // fresh deposit of current positions
-int particles_flush_rho(pic_ctx* c, int s);     // acc -> final/energy mesh, rho +=
+// acc -> final/energy mesh, rho += (from zero with zero_rho) of species s0 .. s0 + ns - 1
+int particles_flush(pic_ctx* c, int s0, int ns, bool zero_rho);
 int particles_push(pic_ctx* c, int s);          // pass1 + scan + pass2 (+deposit)
 int particles_count(pic_ctx* c, int s, int64_t* n);
 int particles_bin_counts(pic_ctx* c, int s, int32_t* dev_counts);

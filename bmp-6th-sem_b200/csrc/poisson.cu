@@ -1064,22 +1064,6 @@ unsigned* arrive_ptr(PoissonState& ps) { return reinterpret_cast<unsigned*>(ps.s
 
 // V-cycle on level 0 (b = r32 -> x = z32) enqueued on stream st; returns
 // the number of kernels launched.
-// Launch with programmatic stream serialisation (see pdl_enter).
-template <typename... P, typename... A>
-void launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
-}
-
 // One V-cycle on st from levels[0].b; the result is in vcycle_out().
 // Returns the number of kernels.  Levels above the fused ones take two
 // kernels each (k_mg_down, k_mg_up); with with_rz the finest k_mg_up also
