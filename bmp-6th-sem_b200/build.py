@@ -19,7 +19,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 def build(debug: bool = False, verbose: bool = False) -> str:
     srcs = [os.path.join(CSRC, s) for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
-    newest = max(os.path.getmtime(p) for p in srcs + [os.path.join(CSRC, "pic_internal.h"),
+    newest = max(os.path.getmtime(p) for p in srcs + [os.path.join(CSRC, "pic_internal.h"), os.path.join(CSRC, "poisson_cluster.cuh"),
                                                           os.path.join(ROOT, "include", "pic_capi.h")])
     if os.path.exists(OUT) and os.path.getmtime(OUT) >= newest and not debug:
         return OUT

@@ -216,9 +216,13 @@ struct PoissonState {
     bool graph_off = false;  // pic_set_poisson_graph(ctx, 0): direct launches
     // exact coarse solve of levels[fused_first] (single contexts; poisson.cu)
     bool direct = false;
-    int direct_nf = 0;
-    float* direct_inv = nullptr;  // [nf][nf] FP32 inverse over the level's free nodes
+    int direct_nf = 0, direct_nfp = 0;  // free nodes; the same rounded up to a multiple of 128
+    float* direct_inv = nullptr;  // [nf][nfp] FP32 inverse over the level's free nodes
     int* direct_free = nullptr;   // level node index of each free node
+    // the cluster solve (poisson_cluster.cuh): its description, empty when the
+    // grid does not fit it
+    std::vector<unsigned char> cluster_desc;
+    size_t cluster_smem = 0;
 };
 
 }  // namespace picb200

@@ -883,7 +883,11 @@ __global__ void __launch_bounds__(kFusedThreads) k_mg_fused(FusedLevels F) {
 // preconditioner stays a valid one for CG.
 constexpr int kDirectMax = 1200;
 
-// inverse of the level's operator over its free nodes (row-major, nf x nf),
+// A row of the inverse in memory, padded with zeros to a multiple of 128: a
+// warp's lane sums columns lane, lane + 32, ..., four of them to a 16-byte load.
+__host__ __device__ __forceinline__ int direct_place(int j) { return (j & ~127) + 4 * (j & 31) + ((j >> 5) & 3); }
+
+// inverse of the level's operator over its free nodes (nf rows in that layout),
 // or false when Cholesky breaks down (not positive definite)
 static bool invert_level(int GX, int GY, double cx, double cy, double cd, const std::vector<uint8_t>& mask,
                          std::vector<int>& freen, std::vector<float>& inv) {
@@ -896,6 +900,7 @@ static bool invert_level(int GX, int GY, double cx, double cy, double cd, const 
             freen.push_back(k);
         }
     const int nf = (int)freen.size();
+    const int nfp = (nf + 127) & ~127;
     std::vector<double> A((size_t)nf * nf, 0.0);
     for (int f = 0; f < nf; ++f) {
         const int k = freen[f];
@@ -934,7 +939,7 @@ static bool invert_level(int GX, int GY, double cx, double cy, double cd, const 
     std::vector<std::vector<int>> below(nf);  // rows k > i with L[k][i] in the envelope
     for (int k = 0; k < nf; ++k)
         for (int i = first[k]; i < k; ++i) below[i].push_back(k);
-    inv.assign((size_t)nf * nf, 0.f);
+    inv.assign((size_t)nf * nfp, 0.f);
     std::vector<double> y(nf), x(nf);
     for (int c = 0; c < nf; ++c) {
         for (int i = 0; i < c; ++i) y[i] = 0.0;
@@ -949,25 +954,36 @@ static bool invert_level(int GX, int GY, double cx, double cy, double cd, const 
             for (int k : below[i]) t -= A[(size_t)k * nf + i] * x[k];
             x[i] = t / A[(size_t)i * nf + i];
         }
-        for (int i = 0; i < nf; ++i) inv[(size_t)i * nf + c] = (float)x[i];
+        for (int i = 0; i < nf; ++i) inv[(size_t)i * nfp + direct_place(c)] = (float)x[i];
     }
     return true;
 }
 
 // x[free_idx[i]] = sum_j inv[i][j] b[free_idx[j]]: a warp a row (lanes over
-// j, then a fixed shuffle tree), b's free values staged in shared memory
+// j, then a fixed shuffle tree), b's free values staged in shared memory.  The first groups of the row are loaded before the wait for
+// the kernel before (the inverse does not change).
 __global__ void __launch_bounds__(256) k_mg_direct(const float* __restrict__ inv, const int* __restrict__ freen,
-                                                   int nf, const float* __restrict__ b, float* __restrict__ x) {
-    extern __shared__ float bs[];
+                                                   int nf, int nfp, const float* __restrict__ b, float* __restrict__ x) {
+    extern __shared__ float4 bs4[];
+    float* bs = reinterpret_cast<float*>(bs4);
+    const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5), n4 = nfp / 4;
+    const float4* row = reinterpret_cast<const float4*>(inv + (int64_t)min(i, nf - 1) * nfp);
+    constexpr int kAhead = 8;  // 1,024 values: nearly the whole row
+    float4 p[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) p[u] = lane + 32 * u < n4 ? __ldg(row + lane + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
     pdl_enter();
-    for (int j = threadIdx.x; j < nf; j += 256) bs[j] = b[freen[j]];
+    for (int j = threadIdx.x; j < nfp; j += 256) bs[direct_place(j)] = j < nf ? b[freen[j]] : 0.f;
     __syncthreads();
-    const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (i >= nf) return;
-    const float* row = inv + (int64_t)i * nf;
     float s = 0.f;
-#pragma unroll 4
-    for (int j = lane; j < nf; j += 32) s = fmaf(row[j], bs[j], s);
+    auto add = [&](const float4& q, const float4& w) {
+        s = fmaf(q.w, w.w, fmaf(q.z, w.z, fmaf(q.y, w.y, fmaf(q.x, w.x, s))));
+    };
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+        if (lane + 32 * u < n4) add(p[u], bs4[lane + 32 * u]);
+    for (int j = lane + 32 * kAhead; j < n4; j += 32) add(__ldg(row + j), bs4[j]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
     if (lane == 0) x[freen[i]] = s;
@@ -996,22 +1012,29 @@ __global__ void k_mg_coarse_mask(const uint8_t* fmask, int fGX, int fGY, uint8_t
 // the first and last column, central elsewhere; E_y central with rows taken
 // modulo GY-1; both on every row.
 
-__device__ __forceinline__ void efield_at(const double* phi, int GX, int GY, double dx, double dy,
-                                          int i, int j, int periodic, double& ex, double& ey) {
+// phi(k): the potential at node k
+template <typename Phi>
+__device__ __forceinline__ void efield_of(const Phi& phi, int GX, int GY, double dx, double dy, int i, int j,
+                                          int periodic, double& ex, double& ey) {
     if (periodic) {
         const int64_t k = (int64_t)j * GX + i;
-        if (i == 0) ex = -((phi[k + 1] - phi[k]) / dx);
-        else if (i == GX - 1) ex = -((phi[k] - phi[k - 1]) / dx);
-        else ex = -((phi[k + 1] - phi[k - 1]) / (2 * dx));
+        if (i == 0) ex = -((phi(k + 1) - phi(k)) / dx);
+        else if (i == GX - 1) ex = -((phi(k) - phi(k - 1)) / dx);
+        else ex = -((phi(k + 1) - phi(k - 1)) / (2 * dx));
         const int P = GY - 1;
         const int ju = j + 1 >= P ? j + 1 - P : j + 1, jd = j == 0 ? P - 1 : j - 1;
-        ey = -((phi[(int64_t)ju * GX + i] - phi[(int64_t)jd * GX + i]) / (2 * dy));
+        ey = -((phi((int64_t)ju * GX + i) - phi((int64_t)jd * GX + i)) / (2 * dy));
         return;
     }
     const int ci = min(max(i, 1), GX - 2), cj = min(max(j, 1), GY - 2);
     const int64_t k = (int64_t)cj * GX + ci;
-    ex = -((phi[k + 1] - phi[k - 1]) / (2 * dx));
-    ey = -((phi[k + GX] - phi[k - GX]) / (2 * dy));
+    ex = -((phi(k + 1) - phi(k - 1)) / (2 * dx));
+    ey = -((phi(k + GX) - phi(k - GX)) / (2 * dy));
+}
+
+__device__ __forceinline__ void efield_at(const double* phi, int GX, int GY, double dx, double dy,
+                                          int i, int j, int periodic, double& ex, double& ey) {
+    efield_of([&](int64_t k) { return phi[k]; }, GX, GY, dx, dy, i, j, periodic, ex, ey);
 }
 
 __global__ void k_efield(const double* phi, const double* bz, int GX, int GY, double dx, double dy,
@@ -1060,6 +1083,8 @@ Grid64 fine_grid(pic_ctx* c) {
     return g;
 }
 
+#include "poisson_cluster.cuh"
+
 unsigned* arrive_ptr(PoissonState& ps) { return reinterpret_cast<unsigned*>(ps.scal + S_COUNT); }
 
 // V-cycle on level 0 (b = r32 -> x = z32) enqueued on stream st; returns
@@ -1074,8 +1099,9 @@ static void enqueue_coarse(pic_ctx* c, cudaStream_t st) {
     PoissonState& ps = c->ps;
     if (ps.direct) {
         const MGLevel& L = ps.levels[ps.fused_first];
-        launch_pdl(k_mg_direct, dim3((unsigned)((ps.direct_nf + 7) / 8)), dim3(256), (size_t)ps.direct_nf * 4, st,
-                   (const float*)ps.direct_inv, (const int*)ps.direct_free, ps.direct_nf, (const float*)L.b, L.x);
+        launch_pdl(k_mg_direct, dim3((unsigned)((ps.direct_nf + 7) / 8)), dim3(256), (size_t)ps.direct_nfp * 4, st,
+                   (const float*)ps.direct_inv, (const int*)ps.direct_free, ps.direct_nf, ps.direct_nfp,
+                   (const float*)L.b, L.x);
     } else {
         launch_pdl(k_mg_fused, dim3(1), dim3(kFusedThreads), ps.fused_smem, st,
                    *reinterpret_cast<const FusedLevels*>(ps.fused_desc));
@@ -1421,6 +1447,7 @@ int poisson_setup(pic_ctx* c) {
         std::vector<float> inv;
         if (invert_level(Lk.GX, Lk.GY, Lk.cx, Lk.cy, Lk.cd, m, freen, inv) && !freen.empty()) {
             ps.direct_nf = (int)freen.size();
+            ps.direct_nfp = (ps.direct_nf + 127) & ~127;
             PIC_CUDA(cudaMalloc(&ps.direct_inv, inv.size() * sizeof(float)));
             PIC_CUDA(cudaMalloc(&ps.direct_free, freen.size() * sizeof(int)));
             PIC_CUDA(cudaMemcpy(ps.direct_inv, inv.data(), inv.size() * sizeof(float), cudaMemcpyHostToDevice));
@@ -1429,6 +1456,30 @@ int poisson_setup(pic_ctx* c) {
         }
     }
     PIC_CUDA(cudaStreamCreateWithFlags(&ps.cap_stream, cudaStreamNonBlocking));
+    ClInst I{};
+    if (ps.direct && cluster_layout(c, I, &ps.cluster_smem) && cluster_supported()) {
+        cluster_describe(c, ps.direct_inv, I);
+        ps.cluster_desc.assign(reinterpret_cast<unsigned char*>(&I), reinterpret_cast<unsigned char*>(&I + 1));
+    }
+    return PIC_OK;
+}
+
+// One solve by the cluster kernel, its scalars left in ps.host_scal too.
+// overwrite: rho still holds the charge density.
+static int enqueue_cluster_solve(pic_ctx* c, bool overwrite) {
+    PoissonState& ps = c->ps;
+    ClInst I;
+    std::memcpy(&I, ps.cluster_desc.data(), sizeof(I));
+    I.tol2 = ps.tol * ps.tol;
+    I.maxit = ps.maxit;
+    I.zero_start = overwrite && (ps.warm == PIC_WARM_ZERO || !ps.have_prev) ? 1 : 0;
+    I.overwrite = overwrite ? 1 : 0;
+    I.host_scal = ps.host_scal;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[1];
+    cluster_config(cfg, at, ps.cluster_smem, c->stream);
+    PIC_CUDA(cudaLaunchKernelEx(&cfg, k_cluster_solve, I));
+    c->launches += 1;
     return PIC_OK;
 }
 
@@ -1474,11 +1525,14 @@ int poisson_solve(pic_ctx* c) {
     PIC_CUDA(cudaEventRecord(ps.ev0, c->stream));
     prof_begin(c, PIC_PHASE_POISSON);
     const bool zero_start = (ps.warm == PIC_WARM_ZERO) || !ps.have_prev;
-    k_overwrite_rho<<<(unsigned)((nodes + 255) / 256), 256, 0, c->stream>>>(
-        nodes, c->mask, c->dir_val, c->rho, c->phi, zero_start ? 1 : 0);
-    c->launches += 1;
     const bool learned = ps.warm == PIC_WARM_LEARNED;
     const bool ws_active = learned || ws_tracking(c);
+    bool cluster = !jacobi && !ps.cluster_desc.empty() && !ps.graph_off;
+    if (!cluster || ws_active) {
+        k_overwrite_rho<<<(unsigned)((nodes + 255) / 256), 256, 0, c->stream>>>(
+            nodes, c->mask, c->dir_val, c->rho, c->phi, zero_start ? 1 : 0);
+        c->launches += 1;
+    }
     if (ws_active) {
         const int guess = ws_before_solve(c, learned && ps.have_prev);
         if (guess < 0) return guess;
@@ -1489,14 +1543,28 @@ int poisson_solve(pic_ctx* c) {
             c->launches += 1;
         }
     }
-    if (!ps.gexec[slot] && !ps.graph_failed) {
-        if (build_graph(c, jacobi) != PIC_OK) ps.graph_failed = true;  // host loop below
-    }
     const double tol2 = ps.tol * ps.tol;
-    int restarts = 0;
+    int restarts = 0, graph_iters = 0;
     double bb = 0, true_rr = 0;
     int status = PIC_OK;
     for (;;) {
+        if (cluster) {
+            PIC_TRY(enqueue_cluster_solve(c, !ws_active));
+            PIC_CUDA(cudaStreamSynchronize(c->stream));
+            bb = ps.host_scal[S_BB];
+            true_rr = ps.host_scal[S_TRUE_RR];
+            if (ps.host_scal[S_STATUS] != 0.0) {
+                status = PIC_ERR_NOT_CONVERGED;
+                break;
+            }
+            if (bb <= 0 || true_rr <= tol2 * bb) break;
+            cluster = false;  // the recursive residual drifted: go on from this iterate below
+            ++restarts;
+            graph_iters = -(int)ps.host_scal[S_IT];
+        }
+        if (!ps.gexec[slot] && !ps.graph_failed) {
+            if (build_graph(c, jacobi) != PIC_OK) ps.graph_failed = true;  // host loop below
+        }
         k_pcg_setup<<<nb, kRedThreads, 0, c->stream>>>(g, c->mask, c->dir_val, c->rho, c->phi,
                                                        ps.r, ps.levels[0].b, ps.partials, nb,
                                                        arrive, ps.scal);
@@ -1542,10 +1610,15 @@ int poisson_solve(pic_ctx* c) {
         ++restarts;
     }
     const int it = (int)ps.host_scal[S_IT];
-    if (ps.gexec[slot] && !ps.graph_off) c->launches += (int64_t)it * ps.body_nodes[slot] + 1;
+    graph_iters += it;
+    if (!cluster && ps.gexec[slot] && !ps.graph_off) c->launches += (int64_t)graph_iters * ps.body_nodes[slot] + 1;
     if (ws_active && status == PIC_OK) PIC_TRY(ws_after_solve(c, c->ws_record));
-    if (c->periodic) PIC_TRY(overwrite_phi(c));  // the last row repeats row 0
-    PIC_TRY(fields_from_phi(c));
+    if (cluster) {
+        c->fields_valid = true;  // the kernel ends with the E field
+    } else {
+        if (c->periodic) PIC_TRY(overwrite_phi(c));  // the last row repeats row 0
+        PIC_TRY(fields_from_phi(c));
+    }
     prof_end(c, PIC_PHASE_POISSON);
     PIC_CUDA(cudaEventRecord(ps.ev1, c->stream));
     PIC_CUDA(cudaStreamSynchronize(c->stream));
