@@ -497,107 +497,225 @@ constexpr int kDownSide = kTileCore + 2 * kDownHalo;
 constexpr int kUpSide = kTileCore + 2 * kUpHalo;
 constexpr int kUpCoarse = kUpSide / 2 + 1;  // coarse nodes under an up tile, a side
 static_assert(kUpHalo % 2 == 0, "up tiles start on an even node");
-constexpr int kTileThreads = 256;      // the finest level's kernels (and r.z)
-constexpr int kTileThreadsSmall = 1024; // levels of fewer tiles than two per SM: shorter chains
+static_assert(kNu == 2, "the tiles' sweeps are written for two");
+constexpr int kTileThreads = 256;  // a tile's threads
 static_assert(kDownSide % 2 == 0 && kUpSide % 2 == 0, "tile rows hold as many nodes of each colour");
 
 // level row of region row j (rows wrap at the level's row count)
 __device__ __forceinline__ int tile_row(int j, int GY) {
-    j %= GY;
-    return j < 0 ? j + GY : j;
-}
-
-// Region nodes a thread loads: all its loads are issued before the first
-// result is used (the load phase is one round trip to memory, not one per
-// node).
-template <int S, int NT>
-constexpr int tile_loads() { return (S * S + NT - 1) / NT; }
-
-// one colour over the region's inner nodes (k_mg_rbgs's arithmetic); region
-// node (li, lj) is level node (i0 + li, j0 + lj), colour (i + j) & 1 (rows
-// wrap only at an even row count, so wrapping keeps the colour)
-template <int S, int NT>
-__device__ __forceinline__ void tile_half_sweep(float* x, const float* b, const uint8_t* m, float cx,
-                                                float cy, float icd, int color, int i0, int j0) {
-    constexpr int HS = S / 2;
-    for (int h = threadIdx.x; h < HS * S; h += NT) {
-        const int lj = h / HS;
-        const int li = 2 * (h - lj * HS) + ((i0 + j0 + lj + color) & 1);
-        const int t = lj * S + li;
-        if (li == 0 || lj == 0 || li == S - 1 || lj == S - 1 || m[t]) continue;
-        const float s = __fmaf_rn(cx, x[t - 1] + x[t + 1], __fmaf_rn(cy, x[t - S] + x[t + S], b[t]));
-        x[t] = s * icd;
+    if ((unsigned)j >= (unsigned)GY) {  // (a division only for rows outside)
+        j %= GY;
+        j = j < 0 ? j + GY : j;
     }
-    __syncthreads();
+    return j;
 }
 
-// level F's smoothing from a zero start, then C.b = restriction of F's residual
-template <int NT>
-__global__ void __launch_bounds__(NT) k_mg_down(LevelDev F, LevelDev C) {
+// A region of side S in shared memory: a row's red nodes ((i + j) even; the
+// regions start where i + j is even), then its black ones, each padded to a
+// multiple of four.  A thread owns a quad: four neighbouring nodes of each
+// colour of one row, kept in its registers with their b and masks, so a half
+// sweep of four nodes is two 16-byte loads (the rows above and below), one
+// word (the neighbour beyond the quad) and a 16-byte store, where the
+// row-major form had seven loads and a store a node with two-way conflicts
+// (a solve from zero to 1e-8, row-major / this: 257^2 nodes 318 / 258 us, 513^2
+// 437 / 326, 1025^2 677 / 512; 256 threads a tile on every level, where levels
+// of few tiles had 1,024).
+// Rows are RS apart so that eight consecutive quads, which may span two rows,
+// cover all banks.
+template <int S>
+struct Region {
+    static constexpr int HW = (S / 2 + 3) & ~3, RS = HW + 32, Q = HW / 4, N = S * RS;
+    static_assert(S * Q <= kTileThreads, "a quad a thread");
+    __device__ __forceinline__ static int at(int li, int lj) {
+        return lj * RS + (((li + lj) & 1) ? HW : 0) + (li >> 1);
+    }
+    // region nodes a thread loads: all its loads are issued before the first
+    // result is used (the load phase is one round trip to memory)
+    static constexpr int NL = (S * S + kTileThreads - 1) / kTileThreads;
+};
+
+struct TileMem {
+    float x[Region<kDownSide>::N], b[Region<kDownSide>::N];
+    uint8_t m[Region<kDownSide>::N];
+    float c[kUpCoarse * kUpCoarse];
+};
+static_assert(Region<kUpSide>::N <= Region<kDownSide>::N, "one buffer for both");
+
+// The barrier of a tile's threads: `bar` 0 is the block's (a tile a block),
+// else a named one.
+__device__ __forceinline__ void tile_sync(int bar) {
+    if (bar == 0) __syncthreads();
+    else asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "n"(kTileThreads) : "memory");
+}
+
+template <int S>
+struct TileQuad {
+    using R = Region<S>;
+    int lj, t;    // its row; index of its first red node
+    bool on, inner;  // it exists; its row is swept (the outer rows and columns keep the halo's outermost values)
+    float4 x[2], b[2];
+    uint32_t m[2];
+
+    __device__ __forceinline__ explicit TileQuad(int tid) {
+        lj = tid / R::Q;
+        t = lj * R::RS + 4 * (tid - lj * R::Q);
+        on = tid < S * R::Q;
+        inner = on && lj > 0 && lj < S - 1;
+    }
+    // west and east neighbours of node n of colour C are o[n + odd - 1] and o[n + odd] of the
+    // other colour's; w[n] = o[n + odd - 1]
+    template <int C>
+    __device__ __forceinline__ void neighbours(const float* sx, float (&w)[5], float4& u, float4& d) const {
+        constexpr int oth = C ? 0 : R::HW;
+        const float4 o = x[1 - C];
+        const bool odd = (lj + C) & 1;
+        const float e = sx[t + oth + (odd ? 4 : -1)];
+        u = *reinterpret_cast<const float4*>(sx + t + oth + R::RS);
+        d = *reinterpret_cast<const float4*>(sx + t + oth - R::RS);
+        w[0] = odd ? o.x : e;
+        w[1] = odd ? o.y : o.x;
+        w[2] = odd ? o.z : o.y;
+        w[3] = odd ? o.w : o.z;
+        w[4] = odd ? e : o.w;
+    }
+    // one colour of Gauss-Seidel (k_mg_rbgs's arithmetic); electrodes stay 0
+    template <int C>
+    __device__ __forceinline__ void sweep(float* sx, float cx, float cy, float icd, int bar) {
+        if (inner) {
+            float w[5];
+            float4 u, d, v;
+            neighbours<C>(sx, w, u, d);
+            v.x = __fmaf_rn(cx, w[0] + w[1], __fmaf_rn(cy, d.x + u.x, b[C].x)) * icd;
+            v.y = __fmaf_rn(cx, w[1] + w[2], __fmaf_rn(cy, d.y + u.y, b[C].y)) * icd;
+            v.z = __fmaf_rn(cx, w[2] + w[3], __fmaf_rn(cy, d.z + u.z, b[C].z)) * icd;
+            v.w = __fmaf_rn(cx, w[3] + w[4], __fmaf_rn(cy, d.w + u.w, b[C].w)) * icd;
+            set<C>(sx, v);
+        }
+        tile_sync(bar);
+    }
+    // x = v where free, 0 at electrodes
+    template <int C>
+    __device__ __forceinline__ void set(float* sx, float4 v) {
+        if (m[C] & 0xffu) v.x = 0.0f;
+        if (m[C] & 0xff00u) v.y = 0.0f;
+        if (m[C] & 0xff0000u) v.z = 0.0f;
+        if (m[C] & 0xff000000u) v.w = 0.0f;
+        x[C] = v;
+        *reinterpret_cast<float4*>(sx + t + (C ? R::HW : 0)) = v;
+    }
+    template <int C>
+    __device__ __forceinline__ void residual(const float* sx, float* sr, float cx, float cy, float cd) const {
+        float w[5];
+        float4 u, d, v;
+        neighbours<C>(sx, w, u, d);
+        v.x = (m[C] & 0xffu) ? 0.0f : mg_residual(b[C].x, x[C].x, w[0], w[1], d.x, u.x, cx, cy, cd);
+        v.y = (m[C] & 0xff00u) ? 0.0f : mg_residual(b[C].y, x[C].y, w[1], w[2], d.y, u.y, cx, cy, cd);
+        v.z = (m[C] & 0xff0000u) ? 0.0f : mg_residual(b[C].z, x[C].z, w[2], w[3], d.z, u.z, cx, cy, cd);
+        v.w = (m[C] & 0xff000000u) ? 0.0f : mg_residual(b[C].w, x[C].w, w[3], w[4], d.w, u.w, cx, cy, cd);
+        *reinterpret_cast<float4*>(sr + t + (C ? R::HW : 0)) = v;
+    }
+};
+
+// The region's nodes this thread loads: their index in the level, -1 outside;
+// their masks (which no kernel of the solve writes: read before the wait for
+// the kernel before).
+template <int S>
+struct TileLoads {
+    int k[Region<S>::NL];
+    uint8_t m[Region<S>::NL];
+    __device__ __forceinline__ TileLoads(const LevelDev& F, int tid, int i0, int j0) {
+#pragma unroll
+        for (int u = 0; u < Region<S>::NL; ++u) {
+            const int t = tid + u * kTileThreads, lj = t / S, i = i0 + t - lj * S;
+            k[u] = (t < S * S && i >= 0 && i < F.GX) ? tile_row(j0 + lj, F.GY) * F.GX + i : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < Region<S>::NL; ++u) m[u] = k[u] < 0 ? 1 : F.mask[k[u]];
+    }
+    // v at the nodes -> the region's array
+    __device__ __forceinline__ static void put(float* to, int tid, const float (&v)[Region<S>::NL]) {
+#pragma unroll
+        for (int u = 0; u < Region<S>::NL; ++u) {
+            const int t = tid + u * kTileThreads, lj = t / S;
+            if (t < S * S) to[Region<S>::at(t - lj * S, lj)] = v[u];
+        }
+    }
+    __device__ __forceinline__ void put_mask(uint8_t* to, int tid) const {
+#pragma unroll
+        for (int u = 0; u < Region<S>::NL; ++u) {
+            const int t = tid + u * kTileThreads, lj = t / S;
+            if (t < S * S) to[Region<S>::at(t - lj * S, lj)] = m[u] ? 1 : 0;
+        }
+        // the padding counts as electrodes
+        constexpr int P = Region<S>::HW - S / 2;
+        if constexpr (P > 0) {
+            for (int t = tid; t < 2 * S * P; t += kTileThreads) {
+                const int half = t / P;
+                to[(half >> 1) * Region<S>::RS + (half & 1) * Region<S>::HW + S / 2 + t - half * P] = 1;
+            }
+        }
+    }
+};
+
+// Tile (bx, by) of level F: its smoothing from a zero start, then C.b = the
+// restriction of F's residual
+template <typename Wait>
+__device__ __forceinline__ void tile_down(const LevelDev& F, const LevelDev& C, int bx, int by, int tid, int bar,
+                                          TileMem& T, const Wait& wait) {
     constexpr int S = kDownSide, H = kDownHalo, CC = kTileCore / 2;
-    __shared__ float sx[S * S], sb[S * S], sr[S * S];
-    __shared__ uint8_t sm[S * S];
-    pdl_enter();
-    const int I0 = blockIdx.x * CC, J0 = blockIdx.y * CC;  // first coarse node of the tile
-    const int i0 = 2 * I0 - H, j0 = 2 * J0 - H;            // level node of region node (0, 0)
+    using R = Region<S>;
+    const int I0 = bx * CC, J0 = by * CC;          // first coarse node of the tile
+    const int i0 = 2 * I0 - H, j0 = 2 * J0 - H;    // level node of region node (0, 0)
+    const int I = I0 + tid % CC, J = J0 + tid / CC;  // the thread's coarse node
+    static_assert(CC * CC == kTileThreads, "a coarse node a thread");
+    const bool cin = I < C.GX && J < C.GY;
+    const uint8_t cm = cin ? C.mask[J * C.GX + I] : 1;
     {
-        constexpr int NL = tile_loads<S, NT>();
-        int kk[NL];
-        uint8_t mv[NL];
-        float bv[NL];
+        const TileLoads<S> L(F, tid, i0, j0);
+        wait();
+        float v[R::NL];
 #pragma unroll
-        for (int u = 0; u < NL; ++u) {
-            const int t = threadIdx.x + u * NT, li = t % S, lj = t / S, i = i0 + li;
-            kk[u] = (t < S * S && i >= 0 && i < F.GX) ? tile_row(j0 + lj, F.GY) * F.GX + i : -1;
-        }
+        for (int u = 0; u < R::NL; ++u) v[u] = L.k[u] < 0 ? 0.0f : F.b[L.k[u]];
+        L.put_mask(T.m, tid);
+        L.put(T.b, tid, v);
+    }
+    tile_sync(bar);
+    TileQuad<S> q(tid);
+    if (q.on) {
 #pragma unroll
-        for (int u = 0; u < NL; ++u) {
-            mv[u] = kk[u] < 0 ? 1 : F.mask[kk[u]];
-            bv[u] = kk[u] < 0 ? 0.0f : F.b[kk[u]];
+        for (int c = 0; c < 2; ++c) {
+            q.b[c] = *reinterpret_cast<const float4*>(T.b + q.t + c * R::HW);
+            q.m[c] = *reinterpret_cast<const uint32_t*>(T.m + q.t + c * R::HW);
         }
+        // zero start: the black sweep reads red x = b / cd (electrodes 0; as a
+        // product with icd, like every update)
+        q.template set<0>(T.x, make_float4(q.b[0].x * F.icd, q.b[0].y * F.icd, q.b[0].z * F.icd, q.b[0].w * F.icd));
+        q.template set<1>(T.x, make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+    tile_sync(bar);
+    q.template sweep<1>(T.x, F.cx, F.cy, F.icd, bar);
+    q.template sweep<0>(T.x, F.cx, F.cy, F.icd, bar);
+    q.template sweep<1>(T.x, F.cx, F.cy, F.icd, bar);
+    if (q.inner) {  // (b is in registers: its array takes the residual)
+        q.template residual<0>(T.x, T.b, F.cx, F.cy, F.cd);
+        q.template residual<1>(T.x, T.b, F.cx, F.cy, F.cd);
+    }
 #pragma unroll
-        for (int u = 0; u < NL; ++u) {
-            const int t = threadIdx.x + u * NT, li = t % S, lj = t / S;
-            if (t >= S * S) break;
-            sm[t] = mv[u];
-            sb[t] = bv[u];
-            // zero start: the black sweep reads red x = b / cd (electrodes 0;
-            // as a product with icd, like every update);
-            // black values are written before anything reads them
-            sx[t] = (!mv[u] && ((i0 + li + j0 + lj) & 1) == 0) ? bv[u] * F.icd : 0.0f;
-        }
+    for (int u = 0; u < kTileCore * kTileCore / kTileThreads; ++u) {
+        const int t = tid + u * kTileThreads, li = H + t % kTileCore, lj = H + t / kTileCore, a = R::at(li, lj);
+        if (!T.m[a] && j0 + lj < F.GY) F.x[(j0 + lj) * F.GX + i0 + li] = T.x[a];
     }
-    __syncthreads();
-    tile_half_sweep<S, NT>(sx, sb, sm, F.cx, F.cy, F.icd, 1, i0, j0);
-    for (int s = 1; s < kNu; ++s) {
-        tile_half_sweep<S, NT>(sx, sb, sm, F.cx, F.cy, F.icd, 0, i0, j0);
-        tile_half_sweep<S, NT>(sx, sb, sm, F.cx, F.cy, F.icd, 1, i0, j0);
-    }
-    for (int t = threadIdx.x; t < S * S; t += NT) {
-        const int li = t % S, lj = t / S;
-        float rv = 0.0f;
-        if (li > 0 && lj > 0 && li < S - 1 && lj < S - 1 && !sm[t])
-            rv = mg_residual(sb[t], sx[t], sx[t - 1], sx[t + 1], sx[t - S], sx[t + S], F.cx, F.cy, F.cd);
-        sr[t] = rv;
-        const int i = i0 + li, j = j0 + lj;
-        if (li >= H && lj >= H && li < H + kTileCore && lj < H + kTileCore && !sm[t] && j < F.GY)
-            F.x[j * F.GX + i] = sx[t];
-    }
-    __syncthreads();
-    // full weighting, in k_mg_restrict's order
-    for (int t = threadIdx.x; t < CC * CC; t += NT) {
-        const int I = I0 + t % CC, J = J0 + t / CC;
-        if (I >= C.GX || J >= C.GY) continue;
-        const int64_t kc = (int64_t)J * C.GX + I;
-        if (C.mask[kc]) {
-            C.b[kc] = 0.0f;
-            continue;
-        }
-        const int c = (2 * J - j0) * S + (2 * I - i0);
-        float s = 4.0f * sr[c];
-        s += 2.0f * (sr[c - 1] + sr[c + 1] + sr[c - S] + sr[c + S]);
-        s += sr[c - S - 1] + sr[c - S + 1] + sr[c + S - 1] + sr[c + S + 1];
-        C.b[kc] = s * 0.0625f;
+    tile_sync(bar);
+    if (cin) {
+        // full weighting, in k_mg_restrict's order; the node is red, as are the
+        // diagonal ones
+        const int a = (H + 2 * (tid / CC)) * R::RS + (H >> 1) + tid % CC;
+        const float *r = T.b + a, *k = r + R::HW;
+        static_assert(H % 2 == 1, "the column west of the node has the next lower half index of neither colour");
+        float s = 4.0f * r[0];
+        s += 2.0f * (k[0] + k[1] + k[-R::RS] + k[R::RS]);
+        s += r[-R::RS] + r[1 - R::RS] + r[R::RS] + r[R::RS + 1];
+        C.b[J * C.GX + I] = cm ? 0.0f : s * 0.0625f;
     }
 }
 
@@ -611,83 +729,111 @@ struct RzArgs {
     double* scal;
 };
 
-
-// xo = level F's x corrected by C.x and smoothed; with kRz also r.z
-template <bool kRz, int NT>
-__global__ void __launch_bounds__(NT) k_mg_up(LevelDev F, LevelDev C, float* xo, RzArgs R) {
-    static_assert(!kRz || NT == kRedThreads, "the r.z reduction is the PCG block reduction");
-    constexpr int S = kUpSide, H = kUpHalo;
-    __shared__ float sx[S * S], sb[S * S], sc[kUpCoarse * kUpCoarse];
-    __shared__ uint8_t sm[S * S];
-    pdl_enter();
-    const int i0 = blockIdx.x * kTileCore - H, j0 = blockIdx.y * kTileCore - H;
+// Tile (bx, by): xo = level F's x corrected by C.x and smoothed; with kRz
+// returns the thread's share of r.z
+template <bool kRz, typename Wait>
+__device__ __forceinline__ double tile_up(const LevelDev& F, const LevelDev& C, float* xo, const double* r, int bx,
+                                          int by, int tid, int bar, TileMem& T, const Wait& wait) {
+    constexpr int S = kUpSide, H = kUpHalo, NC = kTileCore * kTileCore / kTileThreads;
+    using R = Region<S>;
+    const int i0 = bx * kTileCore - H, j0 = by * kTileCore - H;
+    double rv[NC];
     {
-        // the coarse correction's tile first: coarse nodes (i0 / 2 + a,
-        // j0 / 2 + b), rows wrapped like the fine ones (periodic in y the row
-        // counts are even, so (j mod GY) / 2 = (j / 2) mod (GY / 2)); columns
-        // outside the level read 0 (only electrode or outside nodes use them)
-        const int I0 = i0 >> 1, J0 = j0 >> 1;
-        for (int t = threadIdx.x; t < kUpCoarse * kUpCoarse; t += NT) {
-            const int I = I0 + t % kUpCoarse, J = tile_row(J0 + t / kUpCoarse, C.GY);
-            sc[t] = (I >= 0 && I < C.GX) ? C.x[J * C.GX + I] : 0.0f;
-        }
-        // the node's mask, b and x, all loaded before any is used
-        constexpr int NL = tile_loads<S, NT>();
-        int kk[NL];
-        uint8_t mv[NL];
-        float bv[NL], xv[NL];
+        const TileLoads<S> L(F, tid, i0, j0);
+        wait();
+        // the coarse correction's tile: coarse nodes (i0 / 2 + a, j0 / 2 + b),
+        // rows wrapped like the fine ones (periodic in y the row counts are
+        // even, so (j mod GY) / 2 = (j / 2) mod (GY / 2)); columns outside the
+        // level read 0 (only electrode or outside nodes use them)
+        constexpr int NU = (kUpCoarse * kUpCoarse + kTileThreads - 1) / kTileThreads;
+        float cv[NU], bv[R::NL], xv[R::NL];
 #pragma unroll
-        for (int u = 0; u < NL; ++u) {
-            const int t = threadIdx.x + u * NT, i = i0 + t % S;
-            const int j = tile_row(j0 + t / S, F.GY);
-            kk[u] = (t < S * S && i >= 0 && i < F.GX) ? j * F.GX + i : -1;
+        for (int u = 0; u < NU; ++u) {
+            const int t = tid + u * kTileThreads, b = t / kUpCoarse, I = (i0 >> 1) + t - b * kUpCoarse;
+            cv[u] = (t < kUpCoarse * kUpCoarse && I >= 0 && I < C.GX) ? C.x[tile_row((j0 >> 1) + b, C.GY) * C.GX + I] : 0.0f;
         }
 #pragma unroll
-        for (int u = 0; u < NL; ++u) {
-            const bool in = kk[u] >= 0;
-            mv[u] = in ? F.mask[kk[u]] : 1;
-            bv[u] = in ? F.b[kk[u]] : 0.0f;
-            xv[u] = in ? F.x[kk[u]] : 0.0f;
+        for (int u = 0; u < R::NL; ++u) {
+            bv[u] = L.k[u] < 0 ? 0.0f : F.b[L.k[u]];
+            xv[u] = L.k[u] < 0 ? 0.0f : F.x[L.k[u]];
         }
-        __syncthreads();
+        if (kRz) {  // (used after the sweeps)
 #pragma unroll
-        for (int u = 0; u < NL; ++u) {
-            const int t = threadIdx.x + u * NT, li = t % S, lj = t / S, i = i0 + li;
-            if (t >= S * S) break;
-            sm[t] = mv[u];
-            sb[t] = bv[u];
-            float v = xv[u];
-            if (!mv[u]) {
-                // prolonged(): x + the bilinear interpolation of the coarse correction
-                const int j = j0 + lj;
-                const bool ox = i & 1, oy = j & 1;
-                const float* c = sc + ((j >> 1) - J0) * kUpCoarse + ((i >> 1) - I0);
-                float cv;
-                if (!ox && !oy) cv = c[0];
-                else if (ox && !oy) cv = 0.5f * (c[0] + c[1]);
-                else if (!ox && oy) cv = 0.5f * (c[0] + c[kUpCoarse]);
-                else cv = 0.25f * (c[0] + c[1] + c[kUpCoarse] + c[kUpCoarse + 1]);
-                v = xv[u] + cv;
+            for (int u = 0; u < NC; ++u) {
+                const int t = tid + u * kTileThreads, i = bx * kTileCore + t % kTileCore, j = by * kTileCore + t / kTileCore;
+                rv[u] = i < F.GX && j < F.GY ? r[j * F.GX + i] : 0.0;
             }
-            sx[t] = v;
         }
+        L.put_mask(T.m, tid);
+#pragma unroll
+        for (int u = 0; u < NU; ++u)
+            if (tid + u * kTileThreads < kUpCoarse * kUpCoarse) T.c[tid + u * kTileThreads] = cv[u];
+        L.put(T.b, tid, bv);
+        L.put(T.x, tid, xv);
     }
-    __syncthreads();
-    tile_half_sweep<S, NT>(sx, sb, sm, F.cx, F.cy, F.icd, 1, i0, j0);
-    tile_half_sweep<S, NT>(sx, sb, sm, F.cx, F.cy, F.icd, 0, i0, j0);
-    for (int s = 1; s < kNu; ++s) {
-        tile_half_sweep<S, NT>(sx, sb, sm, F.cx, F.cy, F.icd, 1, i0, j0);
-        tile_half_sweep<S, NT>(sx, sb, sm, F.cx, F.cy, F.icd, 0, i0, j0);
+    tile_sync(bar);
+    TileQuad<S> q(tid);
+    if (q.on) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            q.b[c] = *reinterpret_cast<const float4*>(T.b + q.t + c * R::HW);
+            q.m[c] = *reinterpret_cast<const uint32_t*>(T.m + q.t + c * R::HW);
+            q.x[c] = *reinterpret_cast<const float4*>(T.x + q.t + c * R::HW);
+        }
+        // prolonged(): x + the bilinear interpolation of the coarse correction;
+        // columns h .. h + 4 of the coarse row below and the one above.  An
+        // even row's red nodes lie on coarse columns, its black ones between;
+        // an odd row's the other way round.
+        const int oy = q.lj & 1;
+        const float* c0 = T.c + (q.lj >> 1) * kUpCoarse + q.t - q.lj * R::RS;
+        const float* c1 = c0 + kUpCoarse * oy;
+        float lo[5], hi[5];
+#pragma unroll
+        for (int n = 0; n < 5; ++n) {
+            lo[n] = c0[n];
+            hi[n] = c1[n];
+        }
+        float on[4], off[4];  // on a coarse column, between two
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            on[n] = oy ? 0.5f * (lo[n] + hi[n]) : lo[n];
+            off[n] = oy ? 0.25f * (lo[n] + lo[n + 1] + hi[n] + hi[n + 1]) : 0.5f * (lo[n] + lo[n + 1]);
+        }
+        auto add = [](const float4& x, const float (&c)[4]) {
+            return make_float4(x.x + c[0], x.y + c[1], x.z + c[2], x.w + c[3]);
+        };
+        const float4 r4 = oy ? add(q.x[0], off) : add(q.x[0], on), k4 = oy ? add(q.x[1], on) : add(q.x[1], off);
+        q.template set<0>(T.x, r4);
+        q.template set<1>(T.x, k4);
     }
-    double acc[1] = {0.0};
-    for (int t = threadIdx.x; t < kTileCore * kTileCore; t += NT) {
-        const int li = H + t % kTileCore, lj = H + t / kTileCore;
+    tile_sync(bar);
+    q.template sweep<1>(T.x, F.cx, F.cy, F.icd, bar);
+    q.template sweep<0>(T.x, F.cx, F.cy, F.icd, bar);
+    q.template sweep<1>(T.x, F.cx, F.cy, F.icd, bar);
+    q.template sweep<0>(T.x, F.cx, F.cy, F.icd, bar);
+    double acc = 0.0;
+#pragma unroll
+    for (int u = 0; u < NC; ++u) {
+        const int t = tid + u * kTileThreads, li = H + t % kTileCore, lj = H + t / kTileCore, a = R::at(li, lj);
         const int i = i0 + li, j = j0 + lj;
-        if (i >= F.GX || j >= F.GY || sm[lj * S + li]) continue;
-        const float z = sx[lj * S + li];
+        if (j >= F.GY || T.m[a]) continue;
+        const float z = T.x[a];
         xo[j * F.GX + i] = z;
-        if (kRz) acc[0] += R.r[j * F.GX + i] * (double)z;
+        if (kRz) acc += rv[u] * (double)z;
     }
+    return acc;
+}
+
+__global__ void __launch_bounds__(kTileThreads) k_mg_down(LevelDev F, LevelDev C) {
+    __shared__ __align__(16) TileMem T;
+    tile_down(F, C, blockIdx.x, blockIdx.y, threadIdx.x, 0, T, [] { pdl_enter(); });
+}
+
+template <bool kRz>
+__global__ void __launch_bounds__(kTileThreads) k_mg_up(LevelDev F, LevelDev C, float* xo, RzArgs R) {
+    static_assert(kTileThreads == kRedThreads, "the r.z reduction is the PCG block reduction");
+    __shared__ __align__(16) TileMem T;
+    double acc[1] = {tile_up<kRz>(F, C, xo, R.r, blockIdx.x, blockIdx.y, threadIdx.x, 0, T, [] { pdl_enter(); })};
     if (kRz) reduce_finalize<1>(acc, R.partials, gridDim.x * gridDim.y, R.arrive, R.scal, S_RZ);
 }
 
@@ -1108,10 +1254,6 @@ static void enqueue_coarse(pic_ctx* c, cudaStream_t st) {
     }
 }
 
-// fewer tiles than two per SM: blocks of kTileThreadsSmall (the level's time
-// is one block's latency, which more threads a tile shorten)
-static bool small_grid(dim3 g) { return (int64_t)g.x * g.y < 2 * 148; }
-
 int enqueue_vcycle(pic_ctx* c, cudaStream_t st, bool with_rz) {
     PoissonState& ps = c->ps;
     const int kf = ps.fused_first;
@@ -1122,10 +1264,7 @@ int enqueue_vcycle(pic_ctx* c, cudaStream_t st, bool with_rz) {
         const LevelDev C = as_dev(ps.levels[l + 1]);
         const int cc = kTileCore / 2;
         const dim3 grid((C.GX + cc - 1) / cc, (C.GY + cc - 1) / cc);
-        if (small_grid(grid))
-            launch_pdl(k_mg_down<kTileThreadsSmall>, grid, dim3(kTileThreadsSmall), 0, st, F, C);
-        else
-            launch_pdl(k_mg_down<kTileThreads>, grid, tb, 0, st, F, C);
+        launch_pdl(k_mg_down, grid, tb, 0, st, F, C);
         launches += 1;
     }
     enqueue_coarse(c, st);
@@ -1136,13 +1275,10 @@ int enqueue_vcycle(pic_ctx* c, cudaStream_t st, bool with_rz) {
         if (l + 1 < kf) C.x = ps.levels[l + 1].xo;  // what the coarser k_mg_up wrote
         const dim3 grid((F.GX + kTileCore - 1) / kTileCore, (F.GY + kTileCore - 1) / kTileCore);
         if (l == 0 && with_rz)
-            launch_pdl(k_mg_up<true, kTileThreads>, grid, tb, 0, st, F, C, ps.levels[l].xo,
+            launch_pdl(k_mg_up<true>, grid, tb, 0, st, F, C, ps.levels[l].xo,
                        RzArgs{ps.r, ps.partials, arrive_ptr(ps), ps.scal});
-        else if (small_grid(grid))
-            launch_pdl(k_mg_up<false, kTileThreadsSmall>, grid, dim3(kTileThreadsSmall), 0, st, F, C,
-                       ps.levels[l].xo, RzArgs{});
         else
-            launch_pdl(k_mg_up<false, kTileThreads>, grid, tb, 0, st, F, C, ps.levels[l].xo, RzArgs{});
+            launch_pdl(k_mg_up<false>, grid, tb, 0, st, F, C, ps.levels[l].xo, RzArgs{});
         launches += 1;
     }
     return launches;

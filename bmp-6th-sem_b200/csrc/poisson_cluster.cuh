@@ -36,10 +36,11 @@
 
 constexpr int kClBlocks = 16;      // a cluster (non-portable size)
 // Grids up to this many nodes: beyond it the multi-kernel solve, on all SMs, is
-// as fast or faster (measured, us a solve from zero to 1e-8, cluster / kernels:
-// 33^2 nodes 44 / 85, 65^2 152 / 211, 129^2 226 / 265, 161^2 279 / 312, 177^2
-// 299 / 312, 193^2 308 / 311, 101 x 301 328 / 359, 301 x 101 402 / 399).
-constexpr int64_t kClMaxNodes = 32000;
+// as fast or faster.  Measured, us a solve from zero to 1e-8, cluster / kernels:
+// 33^2 nodes 44 / 88, 65^2 153 / 184, 101 x 71 224 / 246, 129^2 225 / 219, 161^2
+// 276 / 250; us a step of a run (host work included): 33^2 83 / 113, 65^2 160 /
+// 190, 97^2 204 / 223, 113^2 213 / 222, 129^2 226 / 222.
+constexpr int64_t kClMaxNodes = 14000;
 constexpr int kClThreads = 1024;
 constexpr int kClMaxLevels = 8;
 constexpr int kClRepNodes = 1500;  // levels up to this size are replicated

@@ -1,8 +1,8 @@
-"""The one-cluster Poisson solve (grids up to 32,000 nodes) against the
+"""The one-cluster Poisson solve (grids up to 14,000 nodes) against the
 multi-kernel solve of the same system (pic_set_poisson_graph(0)): square, odd
 and elongated grids, bands of few and of many rows, an inner electrode,
 periodic in y, levels that are distributed and levels that every block keeps,
-and the first grid too large for it.
+and grids too large for it.
 
 Both are PCG with the same V-cycle, node for node, and alpha and beta are
 summed in the same order, so iterations and potentials are equal to the last
@@ -40,7 +40,7 @@ def _state(pic, s):
     (40, 300, False, True), (300, 40, False, True), (57, 58, False, False), (64, 64, False, True),
     (101, 99, False, True), (128, 128, False, False), (150, 77, False, True), (210, 210, False, True),
     (48, 48, True, False), (90, 64, True, True), (200, 96, True, True), (60, 320, True, False),
-    (7, 300, False, False), (1500, 20, False, False), (177, 177, False, True), (178, 178, False, True),
+    (7, 300, False, False), (1500, 20, False, False), (117, 117, False, True), (118, 118, False, True), (90, 150, True, False),
     (212, 212, False, False),
 ])
 def test_cluster_solve_matches_the_kernels(nx, ny, periodic, inner):
@@ -58,7 +58,8 @@ def test_cluster_solve_matches_the_kernels(nx, ny, periodic, inner):
                 pic.set_rho(rho)
                 pic.poisson_solve(k)
                 it, rel, _ = pic.poisson_stats()
-                assert rel <= 1e-12 and 0 < it < 60
+                # (periodic in y with rows that do not halve twice: one level, hundreds of iterations)
+                assert rel <= 1e-12 and 0 < it < (1000 if periodic and ny % 4 else 60)
                 out.append((it, pic.phi(), pic.rho(), P.Pic.poisson_start_relres(pic)))
             res[graph] = out
         for a, b in zip(res[1], res[0]):
