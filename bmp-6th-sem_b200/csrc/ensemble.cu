@@ -17,6 +17,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <queue>
 #include <vector>
 
 #include "pic_internal.h"
@@ -37,8 +38,10 @@ struct pic_ensemble {
     int* d_active = nullptr;
     int* d_inst_of = nullptr;              // block -> instance of the solve launch
     std::vector<int> blk0, nblk;           // each instance's block range
+    std::vector<int> sum0, nsum;           // the blocks its dot products are summed as
+    double* d_wsum = nullptr;              // their warps' sums
     size_t smem = 0;
-    int blocks = 0;
+    int threads = 0, blocks = 0;
     const double** d_scal_ptrs = nullptr;
     double* d_scal_all = nullptr;
     double* h_scal_all = nullptr;  // pinned
@@ -69,6 +72,7 @@ void free_ensemble(pic_ensemble* e) {
     cudaFree(e->d_insts);
     cudaFree(e->d_fused);
     cudaFree(e->d_partials);
+    cudaFree(e->d_wsum);
     cudaFree(e->d_inst_of);
     cudaFree(e->d_active);
     cudaFree(e->d_scal_ptrs);
@@ -89,7 +93,7 @@ int enqueue_step(pic_ensemble* e, bool capturing) {
     PIC_CUDA(cudaEventRecordWithFlags(e->ev[1], st, evflags));
     PIC_TRY(poisson_batch_launch(e->d_insts, e->n, e->d_inst_of, e->d_partials,
                                  reinterpret_cast<unsigned*>(e->d_active), e->d_active + e->n, e->smem,
-                                 e->blocks, st));
+                                 e->threads, e->blocks, st));
     PIC_CUDA(cudaEventRecordWithFlags(e->ev[2], st, evflags));
     PIC_TRY(batch_push(e->pb, e->shape, e->energy, st));
     PIC_CUDA(cudaEventRecordWithFlags(e->ev[3], st, evflags));
@@ -104,7 +108,7 @@ int upload_poisson(pic_ensemble* e) {
     for (int i = 0; i < e->n; ++i)
         PIC_TRY(poisson_batch_describe(e->cs[i], e->h_insts + (size_t)i * e->desc,
                                        static_cast<char*>(e->d_fused) + (size_t)i * 1024, e->blk0[i],
-                                       e->nblk[i]));
+                                       e->nblk[i], e->nsum[i], e->d_wsum + (size_t)e->sum0[i] * 64));
     PIC_CUDA(cudaMemcpyAsync(e->d_insts, e->h_insts, (size_t)e->n * e->desc, cudaMemcpyHostToDevice,
                              e->stream));
     return PIC_OK;
@@ -143,6 +147,7 @@ int pic_ensemble_create(const pic_config* cfgs, int n, pic_ensemble** out) {
     // batched Poisson: descriptors, fused-level tables, scratch
     e->desc = poisson_batch_desc_bytes();
     size_t smem = 0;
+    int64_t nodes = 0;
     std::vector<char> fused((size_t)n * 1024, 0);
     for (int i = 0; i < n; ++i) {
         size_t fb = 0;
@@ -150,30 +155,47 @@ int pic_ensemble_create(const pic_config* cfgs, int n, pic_ensemble** out) {
         if (fb > 1024) return bail(fail(PIC_ERR_CONFIG, "ensemble: fused-level table too large"));
         std::memcpy(fused.data() + (size_t)i * 1024, f, fb);
         smem = std::max(smem, poisson_fused_smem(e->cs[i]));
+        nodes += e->cs[i]->nodes;
     }
+    int sum_blocks = 0;
+    if ((st = poisson_batch_blocks(nodes, &smem, &e->threads, &e->blocks, &sum_blocks)) != PIC_OK) return bail(st);
     e->smem = smem;
-    if ((st = poisson_batch_blocks(smem, &e->blocks)) != PIC_OK) return bail(st);
-    if (e->blocks < n) return bail(fail(PIC_ERR_CONFIG, "ensemble: more instances than co-resident solver blocks"));
+    if (std::min(e->blocks, sum_blocks) < n) return bail(fail(PIC_ERR_CONFIG, "ensemble: more instances than co-resident solver blocks"));
     std::vector<const double*> scal_ptrs;
     for (auto* c : e->cs) scal_ptrs.push_back(c->ps.scal);
-    // the solve's blocks: at least one per instance, the rest in proportion
-    // to the instances' node counts (largest remainders)
+    // The solve's blocks: one per instance, each further one to the instance
+    // whose blocks then have the most nodes (the solve takes as long as the
+    // slowest one's: of 64 instances of 129^2 .. 385^2 nodes on 148 blocks at most
+    // 36,000 nodes a block, where shares in proportion left 50,000).  Dot products
+    // are summed as by blocks in proportion to the nodes (one each, the rest by
+    // largest remainders): the order that an instance's results go by.
     {
         double total = 0;
         for (auto* c : e->cs) total += (double)c->nodes;
-        e->nblk.assign(n, 1);
-        const int spare = e->blocks - n;
+        e->nsum.assign(n, 1);
+        const int spare = sum_blocks - n;
         std::vector<std::pair<double, int>> rem;
         int given = 0;
         for (int i = 0; i < n; ++i) {
             const double share = spare * (double)e->cs[i]->nodes / total;
             const int whole = (int)share;
-            e->nblk[i] += whole;
+            e->nsum[i] += whole;
             given += whole;
             rem.push_back({share - whole, i});
         }
         std::sort(rem.begin(), rem.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-        for (int k = 0; k < spare - given && k < n; ++k) e->nblk[rem[k].second] += 1;
+        for (int k = 0; k < spare - given && k < n; ++k) e->nsum[rem[k].second] += 1;
+        e->sum0.assign(n, 0);
+        for (int i = 1; i < n; ++i) e->sum0[i] = e->sum0[i - 1] + e->nsum[i - 1];
+        e->nblk.assign(n, 1);
+        std::priority_queue<std::pair<double, int>> most;
+        for (int i = 0; i < n; ++i) most.push({(double)e->cs[i]->nodes, -i});
+        for (int k = n; k < e->blocks; ++k) {
+            const int i = -most.top().second;
+            most.pop();
+            e->nblk[i] += 1;
+            most.push({(double)e->cs[i]->nodes / e->nblk[i], -i});
+        }
         std::vector<int> inst_of((size_t)e->blocks, -1);
         e->blk0.assign(n, 0);
         int b = 0;
@@ -188,6 +210,7 @@ int pic_ensemble_create(const pic_config* cfgs, int n, pic_ensemble** out) {
     if (cudaMallocHost(&e->h_insts, (size_t)n * e->desc) || cudaMalloc(&e->d_insts, (size_t)n * e->desc) ||
         cudaMalloc(&e->d_fused, fused.size()) ||
         cudaMalloc(&e->d_partials, (size_t)e->blocks * 2 * sizeof(double)) ||
+        cudaMalloc(&e->d_wsum, (size_t)(e->sum0[n - 1] + e->nsum[n - 1]) * 64 * sizeof(double)) ||
         cudaMalloc(&e->d_active, (size_t)(n + 1) * sizeof(int)) ||  // barrier counters + error flag
         cudaMalloc(&e->d_scal_ptrs, (size_t)n * sizeof(double*)) ||
         cudaMalloc(&e->d_scal_all, (size_t)n * 16 * sizeof(double)) ||

@@ -343,12 +343,13 @@ int fields_set_bz(pic_ctx* c);
 // batched solve of many contexts (poisson.cu)
 size_t poisson_batch_desc_bytes();
 size_t poisson_batch_max_fused_smem();
-int poisson_batch_describe(pic_ctx* c, void* host_desc, const void* dev_fused, int blk0, int nblk);
+int poisson_batch_describe(pic_ctx* c, void* host_desc, const void* dev_fused, int blk0, int nblk, int sumblk,
+                           double* wsum);
 const void* poisson_fused_table(pic_ctx* c, size_t* bytes);
 size_t poisson_fused_smem(pic_ctx* c);
-int poisson_batch_blocks(size_t smem, int* blocks);
+int poisson_batch_blocks(int64_t nodes, size_t* smem, int* threads, int* blocks, int* sum_blocks);
 int poisson_batch_launch(const void* dev_insts, int n, const int* inst_of, double* partials,
-                         unsigned* barriers, int* err, size_t smem, int blocks, cudaStream_t st);
+                         unsigned* barriers, int* err, size_t smem, int threads, int blocks, cudaStream_t st);
 int poisson_batch_finish(pic_ctx* c, const double* scal, float ms);
 
 }  // namespace picb200

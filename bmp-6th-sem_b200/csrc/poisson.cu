@@ -517,8 +517,8 @@ __device__ __forceinline__ int tile_row(int j, int GY) {
 // sweep of four nodes is two 16-byte loads (the rows above and below), one
 // word (the neighbour beyond the quad) and a 16-byte store, where the
 // row-major form had seven loads and a store a node with two-way conflicts
-// (a solve from zero to 1e-8, row-major / this: 257^2 nodes 318 / 258 us, 513^2
-// 437 / 326, 1025^2 677 / 512; 256 threads a tile on every level, where levels
+// (a solve from zero to 1e-8, row-major / this: 257^2 nodes 318 / 256 us, 513^2
+// 437 / 326, 1025^2 677 / 506; 256 threads a tile on every level, where levels
 // of few tiles had 1,024).
 // Rows are RS apart so that eight consecutive quads, which may span two rows,
 // cover all banks.
@@ -529,17 +529,15 @@ struct Region {
     __device__ __forceinline__ static int at(int li, int lj) {
         return lj * RS + (((li + lj) & 1) ? HW : 0) + (li >> 1);
     }
-    // region nodes a thread loads: all its loads are issued before the first
-    // result is used (the load phase is one round trip to memory)
-    static constexpr int NL = (S * S + kTileThreads - 1) / kTileThreads;
 };
 
-struct TileMem {
+struct alignas(16) TileMem {  // (an array of them keeps the 16-byte loads aligned)
     float x[Region<kDownSide>::N], b[Region<kDownSide>::N];
     uint8_t m[Region<kDownSide>::N];
     float c[kUpCoarse * kUpCoarse];
 };
 static_assert(Region<kUpSide>::N <= Region<kDownSide>::N, "one buffer for both");
+static_assert(sizeof(TileMem) % 16 == 0 && offsetof(TileMem, b) % 16 == 0 && offsetof(TileMem, m) % 16 == 0, "16-byte loads");
 
 // The barrier of a tile's threads: `bar` 0 is the block's (a tile a block),
 // else a named one.
@@ -616,42 +614,49 @@ struct TileQuad {
     }
 };
 
-// The region's nodes this thread loads: their index in the level, -1 outside;
-// their masks (which no kernel of the solve writes: read before the wait for
-// the kernel before).
+// The region's nodes this thread loads: a column, and of it every STEP-th row
+// (an even step: the nodes are of one colour, and their places in the region's
+// arrays a constant apart).  Their index in the level, -1 outside; their masks
+// (which no kernel of the solve writes: read before the wait for the kernel
+// before).
 template <int S>
 struct TileLoads {
-    int k[Region<S>::NL];
-    uint8_t m[Region<S>::NL];
+    using R = Region<S>;
+    static constexpr int STEP = kTileThreads / S & ~1, NL = (S + STEP - 1) / STEP;
+    int a;  // the first node's place, < 0: none
+    int rows;  // how many
+    int k[NL];
+    uint8_t m[NL];
     __device__ __forceinline__ TileLoads(const LevelDev& F, int tid, int i0, int j0) {
+        const int r = tid / S, li = tid - r * S, i = i0 + li;
+        rows = r < STEP ? (S - r + STEP - 1) / STEP : 0;
+        a = R::at(li, r);
+        const bool in = i >= 0 && i < F.GX;
 #pragma unroll
-        for (int u = 0; u < Region<S>::NL; ++u) {
-            const int t = tid + u * kTileThreads, lj = t / S, i = i0 + t - lj * S;
-            k[u] = (t < S * S && i >= 0 && i < F.GX) ? tile_row(j0 + lj, F.GY) * F.GX + i : -1;
-        }
+        for (int u = 0; u < NL; ++u) k[u] = u < rows && in ? tile_row(j0 + r + u * STEP, F.GY) * F.GX + i : -1;
 #pragma unroll
-        for (int u = 0; u < Region<S>::NL; ++u) m[u] = k[u] < 0 ? 1 : F.mask[k[u]];
+        for (int u = 0; u < NL; ++u) m[u] = k[u] < 0 ? 1 : F.mask[k[u]];
     }
-    // v at the nodes -> the region's array
-    __device__ __forceinline__ static void put(float* to, int tid, const float (&v)[Region<S>::NL]) {
+    // the nodes' values of `from`, 0 outside
+    __device__ __forceinline__ void get(const float* from, float (&v)[NL]) const {
 #pragma unroll
-        for (int u = 0; u < Region<S>::NL; ++u) {
-            const int t = tid + u * kTileThreads, lj = t / S;
-            if (t < S * S) to[Region<S>::at(t - lj * S, lj)] = v[u];
-        }
+        for (int u = 0; u < NL; ++u) v[u] = k[u] < 0 ? 0.0f : from[k[u]];
+    }
+    __device__ __forceinline__ void put(float* to, const float (&v)[NL]) const {
+#pragma unroll
+        for (int u = 0; u < NL; ++u)
+            if (u < rows) to[a + u * STEP * R::RS] = v[u];
     }
     __device__ __forceinline__ void put_mask(uint8_t* to, int tid) const {
 #pragma unroll
-        for (int u = 0; u < Region<S>::NL; ++u) {
-            const int t = tid + u * kTileThreads, lj = t / S;
-            if (t < S * S) to[Region<S>::at(t - lj * S, lj)] = m[u] ? 1 : 0;
-        }
+        for (int u = 0; u < NL; ++u)
+            if (u < rows) to[a + u * STEP * R::RS] = m[u] ? 1 : 0;
         // the padding counts as electrodes
-        constexpr int P = Region<S>::HW - S / 2;
+        constexpr int P = R::HW - S / 2;
         if constexpr (P > 0) {
             for (int t = tid; t < 2 * S * P; t += kTileThreads) {
                 const int half = t / P;
-                to[(half >> 1) * Region<S>::RS + (half & 1) * Region<S>::HW + S / 2 + t - half * P] = 1;
+                to[(half >> 1) * R::RS + (half & 1) * R::HW + S / 2 + t - half * P] = 1;
             }
         }
     }
@@ -673,11 +678,10 @@ __device__ __forceinline__ void tile_down(const LevelDev& F, const LevelDev& C, 
     {
         const TileLoads<S> L(F, tid, i0, j0);
         wait();
-        float v[R::NL];
-#pragma unroll
-        for (int u = 0; u < R::NL; ++u) v[u] = L.k[u] < 0 ? 0.0f : F.b[L.k[u]];
+        float v[TileLoads<S>::NL];
+        L.get(F.b, v);
         L.put_mask(T.m, tid);
-        L.put(T.b, tid, v);
+        L.put(T.b, v);
     }
     tile_sync(bar);
     TileQuad<S> q(tid);
@@ -700,10 +704,12 @@ __device__ __forceinline__ void tile_down(const LevelDev& F, const LevelDev& C, 
         q.template residual<0>(T.x, T.b, F.cx, F.cy, F.cd);
         q.template residual<1>(T.x, T.b, F.cx, F.cy, F.cd);
     }
+    {
+        constexpr int D = kTileThreads / kTileCore;  // (even: a thread's nodes are of one colour)
+        const int li = H + tid % kTileCore, lj = H + tid / kTileCore, a = R::at(li, lj), k = (j0 + lj) * F.GX + i0 + li;
 #pragma unroll
-    for (int u = 0; u < kTileCore * kTileCore / kTileThreads; ++u) {
-        const int t = tid + u * kTileThreads, li = H + t % kTileCore, lj = H + t / kTileCore, a = R::at(li, lj);
-        if (!T.m[a] && j0 + lj < F.GY) F.x[(j0 + lj) * F.GX + i0 + li] = T.x[a];
+        for (int u = 0; u < kTileCore / D; ++u)
+            if (!T.m[a + u * D * R::RS] && j0 + lj + u * D < F.GY) F.x[k + u * D * F.GX] = T.x[a + u * D * R::RS];
     }
     tile_sync(bar);
     if (cin) {
@@ -734,7 +740,8 @@ struct RzArgs {
 template <bool kRz, typename Wait>
 __device__ __forceinline__ double tile_up(const LevelDev& F, const LevelDev& C, float* xo, const double* r, int bx,
                                           int by, int tid, int bar, TileMem& T, const Wait& wait) {
-    constexpr int S = kUpSide, H = kUpHalo, NC = kTileCore * kTileCore / kTileThreads;
+    constexpr int S = kUpSide, H = kUpHalo;
+    constexpr int D = kTileThreads / kTileCore, NC = kTileCore / D;  // core nodes a thread: rows D apart (even: of one colour)
     using R = Region<S>;
     const int i0 = bx * kTileCore - H, j0 = by * kTileCore - H;
     double rv[NC];
@@ -746,21 +753,18 @@ __device__ __forceinline__ double tile_up(const LevelDev& F, const LevelDev& C, 
         // even, so (j mod GY) / 2 = (j / 2) mod (GY / 2)); columns outside the
         // level read 0 (only electrode or outside nodes use them)
         constexpr int NU = (kUpCoarse * kUpCoarse + kTileThreads - 1) / kTileThreads;
-        float cv[NU], bv[R::NL], xv[R::NL];
+        float cv[NU], bv[TileLoads<S>::NL], xv[TileLoads<S>::NL];
 #pragma unroll
         for (int u = 0; u < NU; ++u) {
             const int t = tid + u * kTileThreads, b = t / kUpCoarse, I = (i0 >> 1) + t - b * kUpCoarse;
             cv[u] = (t < kUpCoarse * kUpCoarse && I >= 0 && I < C.GX) ? C.x[tile_row((j0 >> 1) + b, C.GY) * C.GX + I] : 0.0f;
         }
-#pragma unroll
-        for (int u = 0; u < R::NL; ++u) {
-            bv[u] = L.k[u] < 0 ? 0.0f : F.b[L.k[u]];
-            xv[u] = L.k[u] < 0 ? 0.0f : F.x[L.k[u]];
-        }
+        L.get(F.b, bv);
+        L.get(F.x, xv);
         if (kRz) {  // (used after the sweeps)
 #pragma unroll
             for (int u = 0; u < NC; ++u) {
-                const int t = tid + u * kTileThreads, i = bx * kTileCore + t % kTileCore, j = by * kTileCore + t / kTileCore;
+                const int i = bx * kTileCore + tid % kTileCore, j = by * kTileCore + tid / kTileCore + u * D;
                 rv[u] = i < F.GX && j < F.GY ? r[j * F.GX + i] : 0.0;
             }
         }
@@ -768,8 +772,8 @@ __device__ __forceinline__ double tile_up(const LevelDev& F, const LevelDev& C, 
 #pragma unroll
         for (int u = 0; u < NU; ++u)
             if (tid + u * kTileThreads < kUpCoarse * kUpCoarse) T.c[tid + u * kTileThreads] = cv[u];
-        L.put(T.b, tid, bv);
-        L.put(T.x, tid, xv);
+        L.put(T.b, bv);
+        L.put(T.x, xv);
     }
     tile_sync(bar);
     TileQuad<S> q(tid);
@@ -812,14 +816,15 @@ __device__ __forceinline__ double tile_up(const LevelDev& F, const LevelDev& C, 
     q.template sweep<1>(T.x, F.cx, F.cy, F.icd, bar);
     q.template sweep<0>(T.x, F.cx, F.cy, F.icd, bar);
     double acc = 0.0;
+    {
+        const int li = H + tid % kTileCore, lj = H + tid / kTileCore, a = R::at(li, lj), k = (j0 + lj) * F.GX + i0 + li;
 #pragma unroll
-    for (int u = 0; u < NC; ++u) {
-        const int t = tid + u * kTileThreads, li = H + t % kTileCore, lj = H + t / kTileCore, a = R::at(li, lj);
-        const int i = i0 + li, j = j0 + lj;
-        if (j >= F.GY || T.m[a]) continue;
-        const float z = T.x[a];
-        xo[j * F.GX + i] = z;
-        if (kRz) acc += rv[u] * (double)z;
+        for (int u = 0; u < NC; ++u) {
+            if (j0 + lj + u * D >= F.GY || T.m[a + u * D * R::RS]) continue;
+            const float z = T.x[a + u * D * R::RS];
+            xo[k + u * D * F.GX] = z;
+            if (kRz) acc += rv[u] * (double)z;
+        }
     }
     return acc;
 }
@@ -859,9 +864,10 @@ struct FusedLevels {
     int mpre[kMaxFused + 1];  // prefix sums of the levels' node counts
 };
 // every thread's share of the masks and of the first level's b, loaded in
-// one round trip (the setup keeps the fused levels within this)
+// one round trip (the setup keeps the fused levels within this for kFusedThreads)
 constexpr int kFusedLoads = 8;
 
+template <int NT>  // the block's threads
 __device__ __forceinline__ void fused_body(const FusedLevels& F, unsigned char* smem) {
     auto X = [&](int l) { return reinterpret_cast<float*>(smem + F.ox[l]); };
     auto B = [&](int l) { return reinterpret_cast<float*>(smem + F.ob[l]); };
@@ -869,23 +875,25 @@ __device__ __forceinline__ void fused_body(const FusedLevels& F, unsigned char* 
     const int tid = threadIdx.x;
     {
         const int n0 = F.GX[0] * F.GY[0], total = F.mpre[F.n];
-        uint8_t mv[kFusedLoads];
-        float bv[kFusedLoads];
-        int lv[kFusedLoads];
+        for (int k0 = tid; k0 < total; k0 += kFusedLoads * NT) {
+            uint8_t mv[kFusedLoads];
+            float bv[kFusedLoads];
+            int lv[kFusedLoads];
 #pragma unroll
-        for (int u = 0; u < kFusedLoads; ++u) {
-            const int k = tid + u * kFusedThreads;
-            int l = 0;
-            while (l + 1 < F.n && k >= F.mpre[l + 1]) ++l;
-            lv[u] = l;
-            mv[u] = k < total ? F.gmask[l][k - F.mpre[l]] : 0;
-            bv[u] = k < n0 ? F.gb[k] : 0.0f;
-        }
+            for (int u = 0; u < kFusedLoads; ++u) {
+                const int k = k0 + u * NT;
+                int l = 0;
+                while (l + 1 < F.n && k >= F.mpre[l + 1]) ++l;
+                lv[u] = l;
+                mv[u] = k < total ? F.gmask[l][k - F.mpre[l]] : 0;
+                bv[u] = k < n0 ? F.gb[k] : 0.0f;
+            }
 #pragma unroll
-        for (int u = 0; u < kFusedLoads; ++u) {
-            const int k = tid + u * kFusedThreads;
-            if (k < total) M(lv[u])[k - F.mpre[lv[u]]] = mv[u];
-            if (k < n0) B(0)[k] = bv[u];
+            for (int u = 0; u < kFusedLoads; ++u) {
+                const int k = k0 + u * NT;
+                if (k < total) M(lv[u])[k - F.mpre[lv[u]]] = mv[u];
+                if (k < n0) B(0)[k] = bv[u];
+            }
         }
     }
     __syncthreads();
@@ -893,7 +901,7 @@ __device__ __forceinline__ void fused_body(const FusedLevels& F, unsigned char* 
     // between the phases (a block barrier of 1024 threads costs more than
     // the few hundred nodes of such a level); the others by the whole block.
     const int ls = F.small;
-    auto stride = [&](int l) { return l >= ls ? 32 : kFusedThreads; };
+    auto stride = [&](int l) { return l >= ls ? 32 : NT; };
     auto sync = [&](int l) {
         if (l >= ls) __syncwarp();
         else __syncthreads();
@@ -1006,14 +1014,14 @@ __device__ __forceinline__ void fused_body(const FusedLevels& F, unsigned char* 
     for (int l = min(ls, last) - 1; l >= 0; --l) up(l);
     {
         const int n = F.GX[0] * F.GY[0];
-        for (int k = tid; k < n; k += kFusedThreads) F.gx[k] = X(0)[k];
+        for (int k = tid; k < n; k += NT) F.gx[k] = X(0)[k];
     }
 }
 
 __global__ void __launch_bounds__(kFusedThreads) k_mg_fused(FusedLevels F) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smem[];
-    fused_body(F, smem);
+    fused_body<kFusedThreads>(F, smem);
 }
 
 // ---- exact solve of the first fused level (single contexts) -------------------
@@ -1829,18 +1837,40 @@ int fields_set_bz(pic_ctx* c) {
 
 // ---------------------------------------------------------------------------
 // Batched solve: the Poisson solves of many instances (an ensemble) in ONE
-// persistent cooperative launch.  Every phase of the PCG iteration and of the
-// V-cycle loops over the instances that are still iterating, each instance's
-// nodes spread over the whole grid, with grid-wide barriers between phases;
-// an instance's fused coarse levels run in one block (block i for instance
-// i).  Dot products are reduced per warp into a per-instance table and
-// summed by one block per instance in fixed order: deterministic.  The solve
-// ends with the true residual and the E field of every instance.
+// persistent cooperative launch.  A share of the blocks works on each instance
+// and meets at the instance's own barriers between the phases of its PCG
+// iterations: a phase a level on the way down and one on the way up
+// (k_mg_down's and k_mg_up's tiles, one for each 256 threads of a block at a
+// time), the fused coarse levels in the instance's first block, and three
+// passes over the FP64 vectors.  Dot products are summed a block, then over
+// the instance's blocks in order, by each of them alike: every block takes the
+// same decisions, and nobody waits for one to have summed.  The solve ends
+// with the true residual and the E field of every instance.
+//
+// What bounds it: the instance whose blocks have the most nodes times
+// iterations, and there the tiles' instructions (60 % of an iteration) and the
+// FP64 passes' bytes (25 %).  64 instances of 128^2 .. 384^2 cells took 4.7 ms
+// with a phase a half sweep (9 barriers a level, a division a node); 4.2 with the
+// tiles, 3.6 with half-SM blocks and even shares, 3.5 with p and A p in one pass.
 // ---------------------------------------------------------------------------
 namespace picb200 {
 namespace {
 
 constexpr int kMaxBatchLevels = 10;
+constexpr int kMaxSumBlocks = 512;  // (an SM a block)
+// Threads of the batch's blocks: 1,024, one block an SM, or 512, two of them.
+// With half-SM blocks the instances' shares come out more even, and one block
+// works while the other waits at a barrier; with whole ones the barriers have
+// half as many blocks and the fused levels, one block's work, twice the
+// threads.
+constexpr int kBatchWhole = 1024, kBatchHalf = 512;
+// Half ones from this many nodes an SM (measured, ms a solve, whole / half:
+// 64 instances of 128^2 .. 384^2 cells, 29,000 nodes an SM, 4.22 / 3.55; 100 of
+// 64^2 .. 256^2, 21,000, 2.53 / 2.31; 24 of 128^2 .. 384^2, 11,000, 2.15 / 1.83;
+// 16 of 256^2 .. 384^2, 11,000, 1.92 / 1.92; 140 of 64^2 .. 128^2, 9,000, 1.19 /
+// 1.21; 3 of 500^2 .. 700^2, 7,000, 1.82 / 1.93; 16 of 64^2 .. 128^2, 0.66 / 0.77).
+constexpr int64_t kBatchHalfNodes = 10000;
+constexpr int kSumWarps = 32;  // of a summing block
 
 struct BatchInst {
     int GX, GY;
@@ -1854,19 +1884,21 @@ struct BatchInst {
     double* rho;  // becomes the right-hand side b
     double* phi;
     double* r;
-    double* z;
-    double* p;
+    double* p[2];  // the direction and the one before, in turn
     double* q;
     const double* bz;
     float4* fld;
     int kf;  // multigrid levels before the fused ones
     LevelDev lev[kMaxBatchLevels];  // levels 0 .. kf
+    float* xo[kMaxBatchLevels];     // the way up's results, levels 0 .. kf - 1
     const FusedLevels* fused;
     double* scal;
     double tol2;
     int maxit;
     int zero_start;
     int blk0, nblk;  // the blocks of the launch that work on this instance
+    int sumblk;      // the blocks that r.z and p.A p are summed as
+    double* wsum;    // their warps' sums, twice
 };
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
@@ -1888,6 +1920,7 @@ struct GroupBarrier {
     unsigned target;
     int nblk;
     int* err;
+    bool given_up;  // thread 0's: a barrier was not met, later ones are not waited for
     __device__ __forceinline__ void sync() {
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -1896,9 +1929,10 @@ struct GroupBarrier {
             atomicAdd(ctr, 1u);
             unsigned polls = 0;
             const unsigned limit = g_spin_limit;
-            while (ld_acquire(ctr) < target) {
+            while (!given_up && ld_acquire(ctr) < target) {
                 if (++polls > limit) {
                     atomicExch(err, 1);
+                    given_up = true;
                     break;
                 }
                 __nanosleep(64);
@@ -1912,47 +1946,71 @@ struct GroupBarrier {
 // Blocks blk0 .. blk0+nblk of the launch work on instance inst_of[block] and
 // meet at the instance's own barriers between phases; each instance iterates
 // until its own convergence.
-__global__ void __launch_bounds__(kFusedThreads) k_poisson_batch(const BatchInst* __restrict__ insts,
+template <int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_poisson_batch(const BatchInst* __restrict__ insts,
                                                                   int n, const int* __restrict__ inst_of,
                                                                   double* partials, unsigned* barriers,
                                                                   int* err) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ double s_red[2][kFusedThreads / 32];
+    __shared__ double s_red[2][NT / 32];
+    __shared__ double s_total;
+    __shared__ double s_blk[kMaxSumBlocks];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int me = inst_of[blockIdx.x];  // -1: a spare block
     if (me < 0) return;
     const BatchInst* I = insts + me;
-    GroupBarrier grid{barriers + me, 0u, I->nblk, err};
+    GroupBarrier grid{barriers + me, 0u, I->nblk, err, false};
     const int64_t ltid = (int64_t)(blockIdx.x - I->blk0) * blockDim.x + threadIdx.x;
     const int64_t lsize = (int64_t)I->nblk * blockDim.x;
     const bool first = blockIdx.x == I->blk0;
 
-    // block sums of two values -> partials[block][0..1]
-    auto put2 = [&](double a, double b) {
+    // the block's sum of a value -> partials[block][slot].  Two slots in turn:
+    // a slot is written again only after a barrier that every block reached
+    // with its reading done.
+    auto put = [&](double a, int slot) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            a += __shfl_xor_sync(kFull, a, o);
-            b += __shfl_xor_sync(kFull, b, o);
-        }
-        if (lane == 0) {
-            s_red[0][warp] = a;
-            s_red[1][warp] = b;
-        }
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
+        if (lane == 0) s_red[slot][warp] = a;
         __syncthreads();
         if (threadIdx.x == 0) {
-            double ta = 0.0, tb = 0.0;
-            for (int w = 0; w < (int)(blockDim.x / 32); ++w) {
-                ta += s_red[0][w];
-                tb += s_red[1][w];
-            }
-            partials[2 * blockIdx.x] = ta;
-            partials[2 * blockIdx.x + 1] = tb;
+            double t = 0.0;
+            for (int w = 0; w < NT / 32; ++w) t += s_red[slot][w];
+            partials[2 * blockIdx.x + slot] = t;
         }
     };
-    // the instance's first block: sum of its blocks' partials, fixed order
-    auto total = [&](int v) {
+    // after a barrier: the sum over the instance's blocks, fixed order
+    auto total = [&](int slot) {
+        if (threadIdx.x == 0) {
+            double t = 0.0;
+#pragma unroll 4
+            for (int b = I->blk0; b < I->blk0 + I->nblk; ++b) t += __ldcg(partials + 2 * b + slot);
+            s_total = t;
+        }
+        __syncthreads();
+        const double t = s_total;
+        __syncthreads();
+        return t;
+    };
+    // a warp's share of an ordered sum: the sum of warp vw of the summing blocks
+    auto put_warp = [&](double a, int slot, int vw) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
+        if (lane == 0) I->wsum[slot * I->sumblk * kSumWarps + vw] = a;
+    };
+    // after a barrier: the summing blocks' warps in order, then those blocks in order
+    auto ordered_total = [&](int slot) {
+        const int sb = I->sumblk;
+        for (int b = threadIdx.x; b < sb; b += NT) {
+            const double* w = I->wsum + ((int64_t)slot * sb + b) * kSumWarps;
+            double t = 0.0;
+#pragma unroll 8
+            for (int n = 0; n < kSumWarps; ++n) t += __ldcg(w + n);
+            s_blk[b] = t;
+        }
+        __syncthreads();
         double t = 0.0;
-        for (int b = I->blk0; b < I->blk0 + I->nblk; ++b) t += partials[2 * b + v];
+        for (int b = 0; b < sb; ++b) t += s_blk[b];
+        __syncthreads();
         return t;
     };
     auto stencil64 = [&](const double* x, int64_t k) {
@@ -1961,219 +2019,150 @@ __global__ void __launch_bounds__(kFusedThreads) k_poisson_batch(const BatchInst
     };
 
     // overwriteRho and the electrode potentials (zero start: phi = 0 elsewhere)
-    if (I) {
-        for (int64_t k = ltid; k < I->nodes; k += lsize) {
-            if (I->mask[k]) {
-                I->rho[k] = -I->dv[k];
-                I->phi[k] = I->dv[k];
-            } else {
-                I->rho[k] = -I->rho[k];
-                if (I->zero_start) I->phi[k] = 0.0;
-            }
+    for (int64_t k = ltid; k < I->nodes; k += lsize) {
+        if (I->mask[k]) {
+            I->rho[k] = -I->dv[k];
+            I->phi[k] = I->dv[k];
+        } else {
+            I->rho[k] = -I->rho[k];
+            if (I->zero_start) I->phi[k] = 0.0;
         }
     }
     grid.sync();
     // r = b - A x, MG input r32; |r|^2 and |b_red|^2
-    if (I) {
-        double rr = 0.0, bb = 0.0;
-        for (int64_t k = ltid; k < I->sn; k += lsize) {
-            double ri = 0.0;
-            if (!I->mask[k]) {
-                ri = I->rho[k] - stencil64(I->phi, k);
-                const double br = I->rho[k] + I->cx * (dirv(I->mask, I->dv, k - 1) + dirv(I->mask, I->dv, k + 1)) +
-                                  I->cy * (dirv(I->mask, I->dv, row_dn(k, I->sn, I->GX)) +
-                                           dirv(I->mask, I->dv, row_up(k, I->sn, I->GX)));
-                bb += br * br;
-            }
-            I->r[k] = ri;
-            I->lev[0].b[k] = (float)ri;
-            rr += ri * ri;
+    double rr = 0.0, bb = 0.0;
+    for (int64_t k = ltid; k < I->sn; k += lsize) {
+        double ri = 0.0;
+        if (!I->mask[k]) {
+            ri = I->rho[k] - stencil64(I->phi, k);
+            const double br = I->rho[k] + I->cx * (dirv(I->mask, I->dv, k - 1) + dirv(I->mask, I->dv, k + 1)) +
+                              I->cy * (dirv(I->mask, I->dv, row_dn(k, I->sn, I->GX)) +
+                                       dirv(I->mask, I->dv, row_up(k, I->sn, I->GX)));
+            bb += br * br;
         }
-        put2(rr, bb);
+        I->r[k] = ri;
+        I->lev[0].b[k] = (float)ri;
+        rr += ri * ri;
     }
+    put(rr, 0);
+    put(bb, 1);
     grid.sync();
-    if (first && threadIdx.x == 0) {
-        const double rr = total(0), bb = total(1);
-        I->scal[S_RR] = rr;
-        I->scal[S_BB] = bb;
-        I->scal[S_RZ_OLD] = 0.0;
-        I->scal[S_IT] = 0.0;
-        I->scal[S_STATUS] = 0.0;
-        I->scal[S_COUNT] = (bb > 0.0 && rr > I->tol2 * bb) ? 1.0 : 0.0;  // go on
-    }
-    grid.sync();
-    const int maxkf = I->kf;
-    for (int it = 0; it < I->maxit; ++it) {
-        if (I->scal[S_COUNT] == 0.0) break;  // the same value for all the instance's blocks
-        const bool on = true;
-        // ---- V-cycle: levels above the fused ones ----
-        // one colour of a Gauss-Seidel sweep; four nodes per thread and
-        // round, their loads issued before their stores (memory-level
-        // parallelism: one block per SM)
-        auto half_sweep = [&](int l, int color) {
-            if (on && l < I->kf) {
-                const LevelDev& L = I->lev[l];
-                const int hw = (L.GX + 1) >> 1, n = hw * L.GY, ls = (int)lsize, nl = L.GX * L.GY;
-                for (int h0 = (int)ltid; h0 < n; h0 += 4 * ls) {
-                    int k[4];
-                    bool ok[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int h = h0 + u * ls;
-                        const int j = h / hw;
-                        const int x = 2 * (h - j * hw) + ((j + color) & 1);
-                        k[u] = j * L.GX + x;
-                        ok[u] = h < n && x < L.GX;
-                        ok[u] = ok[u] && !L.mask[k[u]];
-                    }
-                    float v[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        v[u] = ok[u] ? __fmaf_rn(L.cx, L.x[k[u] - 1] + L.x[k[u] + 1],
-                                                 __fmaf_rn(L.cy, L.x[row_dn(k[u], nl, L.GX)] + L.x[row_up(k[u], nl, L.GX)],
-                                                           L.b[k[u]]))
-                                     : 0.0f;
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (ok[u]) L.x[k[u]] = v[u] * L.icd;
-                }
-            }
-            grid.sync();
-        };
-        // the first black sweep fused with the zero start (mode 0) or with
-        // the coarse correction (mode 1): each black node computes its red
-        // neighbours' values itself (as k_mg_init_black / k_mg_prolong_black)
-        auto first_black = [&](int l, int mode) {
-            if (on && l < I->kf) {
-                const LevelDev& L = I->lev[l];
-                const LevelDev& C = I->lev[l + 1];
-                const int hw = (L.GX + 1) >> 1, n = hw * L.GY, ls = (int)lsize, nl = L.GX * L.GY;
-                for (int h = (int)ltid; h < n; h += ls) {
-                    const int j = h / hw;
-                    const int x = 2 * (h - j * hw) + ((j + 1) & 1);
-                    if (x >= L.GX) continue;
-                    const int k = j * L.GX + x;
-                    if (L.mask[k]) continue;
-                    float w, e, d, u;
-                    if (mode == 0) {
-                        auto xr = [&](int m) { return L.mask[m] ? 0.0f : L.b[m] * L.icd; };
-                        w = xr(k - 1);
-                        e = xr(k + 1);
-                        d = xr(row_dn(k, nl, L.GX));
-                        u = xr(row_up(k, nl, L.GX));
-                    } else {
-                        const int jd = j == 0 ? L.GY - 1 : j - 1, ju = j + 1 == L.GY ? 0 : j + 1;
-                        w = prolonged(L, C, x - 1, j);
-                        e = prolonged(L, C, x + 1, j);
-                        d = prolonged(L, C, x, jd);
-                        u = prolonged(L, C, x, ju);
-                    }
-                    L.x[k] = __fmaf_rn(L.cx, w + e, __fmaf_rn(L.cy, d + u, L.b[k])) * L.icd;
-                }
-            }
-            grid.sync();
-        };
-        for (int l = 0; l < maxkf; ++l) {
-            first_black(l, 0);
-            for (int s = 1; s < kNu; ++s) {
-                half_sweep(l, 0);
-                half_sweep(l, 1);
-            }
-            if (on && l < I->kf) {
-                const LevelDev& F = I->lev[l];
-                const LevelDev& C = I->lev[l + 1];
-                const int nc = C.GX * C.GY;
-#pragma unroll 4
-                for (int kc = (int)ltid; kc < nc; kc += (int)lsize) {
-                    if (C.mask[kc]) {
-                        C.b[kc] = 0.0f;
-                        continue;
-                    }
-                    const int jc = kc / C.GX;
-                    const int x = 2 * (kc - jc * C.GX), j = 2 * jc;
-                    float s = 4.0f * fine_residual(F, x, j);
-                    s += 2.0f * (fine_residual(F, x - 1, j) + fine_residual(F, x + 1, j) +
-                                 fine_residual(F, x, j - 1) + fine_residual(F, x, j + 1));
-                    s += fine_residual(F, x - 1, j - 1) + fine_residual(F, x + 1, j - 1) +
-                         fine_residual(F, x - 1, j + 1) + fine_residual(F, x + 1, j + 1);
-                    C.b[kc] = s * 0.0625f;
-                }
+    rr = total(0);
+    bb = total(1);
+    double rz_old = 0.0;
+    int it = 0, status = 0;
+    bool go = bb > 0.0 && rr > I->tol2 * bb && I->maxit > 0;
+    const int kf = I->kf;
+    // the tiles this block's groups of threads take: one in `groups` of the instance's
+    const int grp = threadIdx.x / kTileThreads, gt = threadIdx.x % kTileThreads;
+    const int group = (blockIdx.x - I->blk0) * (NT / kTileThreads) + grp, groups = I->nblk * (NT / kTileThreads);
+    TileMem& T = reinterpret_cast<TileMem*>(smem)[grp];
+    const uint8_t* __restrict__ mk = I->mask;
+    const float* __restrict__ z = kf > 0 ? I->xo[0] : I->lev[0].x;
+    const int nn = (int)I->sn, GX = I->GX;
+    const double cd = I->cd, cx = I->cx, cy = I->cy;
+    // the summing blocks' threads and warps; the first of this warp's, spread over the blocks
+    const int vws = I->sumblk * kSumWarps, vsize = 32 * vws, vwn = I->nblk * (NT / 32);
+    const int vw0 = (int)(blockIdx.x - I->blk0) + I->nblk * warp;
+    while (go) {
+        // ---- V-cycle ----
+        for (int l = 0; l < kf; ++l) {
+            const LevelDev F = I->lev[l], C = I->lev[l + 1];
+            constexpr int cc = kTileCore / 2;
+            const int tx = (C.GX + cc - 1) / cc, n = tx * ((C.GY + cc - 1) / cc);
+            for (int t = group; t < n; t += groups) {
+                const int by = t / tx;
+                tile_down(F, C, t - by * tx, by, gt, 1 + grp, T, [] {});
+                tile_sync(1 + grp);
             }
             grid.sync();
         }
-        if (on && first) fused_body(*I->fused, smem);
+        if (first) fused_body<NT>(*I->fused, smem);
         grid.sync();
-        for (int l = maxkf - 1; l >= 0; --l) {
-            first_black(l, 1);
-            half_sweep(l, 0);
-            for (int s = 1; s < kNu; ++s) {
-                half_sweep(l, 1);
-                half_sweep(l, 0);
+        for (int l = kf - 1; l >= 0; --l) {
+            const LevelDev F = I->lev[l];
+            LevelDev C = I->lev[l + 1];
+            if (l + 1 < kf) C.x = I->xo[l + 1];
+            const int tx = (F.GX + kTileCore - 1) / kTileCore, n = tx * ((F.GY + kTileCore - 1) / kTileCore);
+            for (int t = group; t < n; t += groups) {
+                const int by = t / tx;
+                tile_up<false>(F, C, I->xo[l], nullptr, t - by * tx, by, gt, 1 + grp, T, [] {});
+                tile_sync(1 + grp);
             }
+            grid.sync();
         }
         // ---- PCG update ----
-        if (on) {
-            double rz = 0.0;
-            const float* __restrict__ x0 = I->lev[0].x;
+        // r.z.  Its order, like that of p.A p below, belongs to sumblk blocks of
+        // 1,024 threads (sums of another order end in other last bits, which a
+        // run's particles amplify), whose warps the instance's warps take in turn
+        for (int vw = vw0; vw < vws; vw += vwn) {
+            double a = 0.0;
             const double* __restrict__ rv = I->r;
-            double* __restrict__ zv = I->z;
-            const uint8_t* __restrict__ mk = I->mask;
-            const int nn = (int)I->sn;
-#pragma unroll 4
-            for (int k = (int)ltid; k < nn; k += (int)lsize) {
-                const double zi = mk[k] ? 0.0 : (double)x0[k];
-                zv[k] = zi;
-                rz += rv[k] * zi;
+            for (int k0 = 32 * vw + lane; k0 < nn; k0 += 8 * vsize) {
+                double r[8];
+                float zk[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int k = k0 + u * vsize;
+                    const bool in = k < nn;
+                    r[u] = in ? rv[k] : 0.0;
+                    zk[u] = in && !mk[k] ? z[k] : 0.0f;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) a += r[u] * (double)zk[u];
             }
-            put2(rz, 0.0);
+            put_warp(a, 0, vw);
         }
         grid.sync();
-        if (on && first && threadIdx.x == 0) I->scal[S_RZ] = total(0);
-        grid.sync();
-        if (on) {
-            const double ro = I->scal[S_RZ_OLD];
-            const double beta = ro == 0.0 ? 0.0 : I->scal[S_RZ] / ro;
-            const double* __restrict__ zv = I->z;
-            double* __restrict__ pv = I->p;
-            const uint8_t* __restrict__ mk = I->mask;
-            const int nn = (int)I->sn;
-#pragma unroll 4
-            // (the first iteration does not read p: what a solve that gave up
-            // left there, NaN included, never reaches the next one)
-            for (int k = (int)ltid; k < nn; k += (int)lsize)
-                pv[k] = mk[k] ? 0.0 : (beta == 0.0 ? zv[k] : zv[k] + beta * pv[k]);
-        }
-        grid.sync();
-        if (on) {
-            double pq = 0.0;
-            const double* __restrict__ pv = I->p;
+        const double rz = ordered_total(0);
+        // p = z + beta p_old, at a node and its neighbours alike (a pass and a
+        // barrier less than p first and then A p; p_old is in the other array),
+        // q = A p, and their product.  The first iteration does not read p_old:
+        // what a solve that gave up left there, NaN included, never reaches the
+        // next one.  (z and p are 0 at electrodes.)
+        const double beta = rz_old == 0.0 ? 0.0 : rz / rz_old;
+        for (int vw = vw0; vw < vws; vw += vwn) {
+            double a = 0.0;
+            const double* __restrict__ po = I->p[it & 1];
+            double* __restrict__ pv = I->p[(it & 1) ^ 1];
             double* __restrict__ qv = I->q;
-            const uint8_t* __restrict__ mk = I->mask;
-            const int nn = (int)I->sn, GX = I->GX;
-            const double cd = I->cd, cx = I->cx, cy = I->cy;
-#pragma unroll 4
-            for (int k = (int)ltid; k < nn; k += (int)lsize) {
-                const double qi = mk[k] ? 0.0
-                                        : cd * pv[k] - cx * (pv[k - 1] + pv[k + 1]) -
-                                              cy * (pv[row_dn(k, nn, GX)] + pv[row_up(k, nn, GX)]);
-                qv[k] = qi;
-                pq += pv[k] * qi;
+            for (int k0 = 32 * vw + lane; k0 < nn; k0 += 2 * vsize) {
+                double c[2][5];
+                float zk[2][5];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int k = k0 + u * vsize;
+                    const bool in = k < nn && !mk[k], old = in && beta != 0.0;
+                    const int at[5] = {k, in ? k - 1 : k, in ? k + 1 : k, in ? row_dn(k, nn, GX) : k, in ? row_up(k, nn, GX) : k};
+#pragma unroll
+                    for (int n = 0; n < 5; ++n) {
+                        zk[u][n] = in ? z[at[n]] : 0.0f;
+                        c[u][n] = old ? po[at[n]] : 0.0;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int k = k0 + u * vsize;
+                    if (k >= nn) break;
+#pragma unroll
+                    for (int n = 0; n < 5; ++n) c[u][n] = (double)zk[u][n] + beta * c[u][n];
+                    const double qi = cd * c[u][0] - cx * (c[u][1] + c[u][2]) - cy * (c[u][3] + c[u][4]);
+                    pv[k] = c[u][0];
+                    qv[k] = qi;
+                    a += c[u][0] * qi;
+                }
             }
-            put2(pq, 0.0);
+            put_warp(a, 1, vw);
         }
         grid.sync();
-        if (on && first && threadIdx.x == 0) I->scal[S_PQ] = total(0);
-        grid.sync();
-        if (on) {
-            const double alpha = I->scal[S_RZ] / I->scal[S_PQ];
-            double rr = 0.0;
-            const double* __restrict__ pv = I->p;
+        const double alpha = rz / ordered_total(1);
+        {
+            double a = 0.0;
+            const double* __restrict__ pv = I->p[(it & 1) ^ 1];
             const double* __restrict__ qv = I->q;
             double* __restrict__ xv = I->phi;
             double* __restrict__ rv = I->r;
             float* __restrict__ b0 = I->lev[0].b;
-            const uint8_t* __restrict__ mk = I->mask;
-            const int nn = (int)I->sn;
 #pragma unroll 4
             for (int k = (int)ltid; k < nn; k += (int)lsize) {
                 double ri = 0.0;
@@ -2183,42 +2172,40 @@ __global__ void __launch_bounds__(kFusedThreads) k_poisson_batch(const BatchInst
                 }
                 rv[k] = ri;
                 b0[k] = (float)ri;
-                rr += ri * ri;
+                a += ri * ri;
             }
-            put2(rr, 0.0);
+            put(a, 0);
         }
         grid.sync();
-        if (on && first && threadIdx.x == 0) {
-            const double rr = total(0);
-            const double its = I->scal[S_IT] + 1.0;
-            I->scal[S_IT] = its;
-            I->scal[S_RZ_OLD] = I->scal[S_RZ];
-            I->scal[S_RR] = rr;
-            const bool finite = isfinite(rr);
-            bool go = finite && rr > I->tol2 * I->scal[S_BB];
-            if (go && its >= (double)I->maxit) {
-                go = false;
-                I->scal[S_STATUS] = 1.0;
-            }
-            if (!finite) I->scal[S_STATUS] = 2.0;
-            I->scal[S_COUNT] = go ? 1.0 : 0.0;
+        rr = total(0);
+        rz_old = rz;
+        ++it;
+        const bool finite = isfinite(rr);
+        go = finite && rr > I->tol2 * bb;
+        if (go && it >= I->maxit) {
+            go = false;
+            status = 1;
         }
-        grid.sync();
+        if (!finite) status = 2;
     }
-    // true residual of every instance, then its E field
-    if (I) {
-        double rr = 0.0;
+    // the true residual, then the E field
+    {
+        double a = 0.0;
         for (int64_t k = ltid; k < I->sn; k += lsize) {
             if (I->mask[k]) continue;
             const double ri = I->rho[k] - stencil64(I->phi, k);
-            rr += ri * ri;
+            a += ri * ri;
         }
-        put2(rr, 0.0);
+        put(a, 1);
     }
     grid.sync();
+    const double true_rr = total(1);
     if (first && threadIdx.x == 0) {
-        I->scal[S_TRUE_RR] = total(0);
-        if (*err) I->scal[S_STATUS] = 3.0;
+        I->scal[S_RR] = rr;
+        I->scal[S_BB] = bb;
+        I->scal[S_IT] = (double)it;
+        I->scal[S_TRUE_RR] = true_rr;
+        I->scal[S_STATUS] = *(volatile int*)err ? 3.0 : (double)status;
     }
     if (I->periodic) {
         // overwritePhi: the last row repeats row 0 (final, electrodes
@@ -2228,13 +2215,11 @@ __global__ void __launch_bounds__(kFusedThreads) k_poisson_batch(const BatchInst
             I->phi[last + i] = I->mask[last + i] ? I->dv[last + i] : I->phi[i];
         grid.sync();
     }
-    if (I) {
-        for (int64_t k = ltid; k < I->nodes; k += lsize) {
-            const int x = (int)(k % I->GX), j = (int)(k / I->GX);
-            double ex, ey;
-            efield_at(I->phi, I->GX, I->GY, I->dx, I->dy, x, j, I->periodic, ex, ey);
-            I->fld[k] = make_float4((float)ex, (float)ey, (float)I->bz[k], 0.0f);
-        }
+    for (int64_t k = ltid; k < I->nodes; k += lsize) {
+        const int x = (int)(k % I->GX), j = (int)(k / I->GX);
+        double ex, ey;
+        efield_at(I->phi, I->GX, I->GY, I->dx, I->dy, x, j, I->periodic, ex, ey);
+        I->fld[k] = make_float4((float)ex, (float)ey, (float)I->bz[k], 0.0f);
     }
 }
 
@@ -2245,7 +2230,8 @@ __global__ void __launch_bounds__(kFusedThreads) k_poisson_batch(const BatchInst
 size_t poisson_batch_desc_bytes() { return sizeof(BatchInst); }
 size_t poisson_batch_max_fused_smem() { return 64 * 1024 + 1024; }
 
-int poisson_batch_describe(pic_ctx* c, void* host_desc, const void* dev_fused, int blk0, int nblk) {
+int poisson_batch_describe(pic_ctx* c, void* host_desc, const void* dev_fused, int blk0, int nblk, int sumblk,
+                           double* wsum) {
     PoissonState& ps = c->ps;
     if (ps.fused_first + 1 > kMaxBatchLevels) return fail(PIC_ERR_CONFIG, "too many multigrid levels for the batched solve");
     if (ps.warm == PIC_WARM_LEARNED) return fail(PIC_ERR_CONFIG, "the batched solve has no learned warm start");
@@ -2268,13 +2254,16 @@ int poisson_batch_describe(pic_ctx* c, void* host_desc, const void* dev_fused, i
     I.rho = c->rho;
     I.phi = c->phi;
     I.r = ps.r;
-    I.z = ps.z;
-    I.p = ps.p[0];
+    I.p[0] = ps.p[0];
+    I.p[1] = ps.p[1];
     I.q = ps.q;
     I.bz = c->bz;
     I.fld = c->fld;
     I.kf = ps.fused_first;
-    for (int l = 0; l <= ps.fused_first; ++l) I.lev[l] = as_dev(ps.levels[l]);
+    for (int l = 0; l <= ps.fused_first; ++l) {
+        I.lev[l] = as_dev(ps.levels[l]);
+        I.xo[l] = ps.levels[l].xo;
+    }
     I.fused = static_cast<const FusedLevels*>(dev_fused);
     I.scal = ps.scal;
     I.tol2 = ps.tol * ps.tol;
@@ -2282,6 +2271,8 @@ int poisson_batch_describe(pic_ctx* c, void* host_desc, const void* dev_fused, i
     I.zero_start = (ps.warm == PIC_WARM_ZERO || !ps.have_prev) ? 1 : 0;
     I.blk0 = blk0;
     I.nblk = nblk;
+    I.sumblk = sumblk;
+    I.wsum = wsum;
     std::memcpy(host_desc, &I, sizeof(I));
     return PIC_OK;
 }
@@ -2294,15 +2285,18 @@ const void* poisson_fused_table(pic_ctx* c, size_t* bytes) {
 
 size_t poisson_fused_smem(pic_ctx* c) { return c->ps.fused_smem; }
 
+static const void* batch_kernel(int threads) {
+    return threads == kBatchHalf ? (const void*)k_poisson_batch<kBatchHalf> : (const void*)k_poisson_batch<kBatchWhole>;
+}
+
 int poisson_batch_launch(const void* dev_insts, int n, const int* inst_of, double* partials,
-                         unsigned* barriers, int* err, size_t smem, int blocks, cudaStream_t st) {
+                         unsigned* barriers, int* err, size_t smem, int threads, int blocks, cudaStream_t st) {
     // the barriers' arrival counters start at zero
     PIC_CUDA(cudaMemsetAsync(barriers, 0, (size_t)n * sizeof(unsigned), st));
     PIC_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
     void* args[] = {(void*)&dev_insts, (void*)&n, (void*)&inst_of, (void*)&partials, (void*)&barriers,
                     (void*)&err};
-    PIC_CUDA(cudaLaunchCooperativeKernel((const void*)k_poisson_batch, dim3(blocks), dim3(kFusedThreads),
-                                         args, smem, st));
+    PIC_CUDA(cudaLaunchCooperativeKernel(batch_kernel(threads), dim3(blocks), dim3(threads), args, smem, st));
     return PIC_OK;
 }
 
@@ -2314,16 +2308,23 @@ int poisson_set_spin_limit(int64_t polls) {
     return PIC_OK;
 }
 
-int poisson_batch_blocks(size_t smem, int* blocks) {
-    cudaFuncAttributes fa{};  // (grows only: other ensembles may be alive)
-    PIC_CUDA(cudaFuncGetAttributes(&fa, k_poisson_batch));
-    if ((int)smem > fa.maxDynamicSharedSizeBytes)
-        PIC_CUDA(cudaFuncSetAttribute(k_poisson_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+// The launch of the batched solve of instances with `nodes` nodes in all: threads and number of its
+// blocks, their shared memory (in: what the fused levels need) and the number
+// of summing blocks.
+int poisson_batch_blocks(int64_t nodes, size_t* smem, int* threads, int* blocks, int* sum_blocks) {
     int per_sm = 0, dev = 0, sms = 0;
-    PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_poisson_batch, kFusedThreads, smem));
     PIC_CUDA(cudaGetDevice(&dev));
     PIC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    *blocks = per_sm * sms;
+    *threads = nodes >= kBatchHalfNodes * sms ? kBatchHalf : kBatchWhole;
+    *smem = std::max(*smem, *threads / kTileThreads * sizeof(TileMem));
+    const void* kernel = batch_kernel(*threads);
+    cudaFuncAttributes fa{};  // (grows only: other ensembles may be alive)
+    PIC_CUDA(cudaFuncGetAttributes(&fa, kernel));
+    if ((int)*smem > fa.maxDynamicSharedSizeBytes)
+        PIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem));
+    PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, *threads, *smem));
+    *blocks = std::min(per_sm, kBatchWhole / *threads) * sms;
+    *sum_blocks = std::min(sms, kMaxSumBlocks);
     if (*blocks <= 0) return fail(PIC_ERR_CONFIG, "the batched solve does not fit on the device");
     return PIC_OK;
 }
