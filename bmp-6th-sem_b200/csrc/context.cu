@@ -41,9 +41,9 @@ static int check_species(pic_ctx* c, int s) {
 // ---------------------------------------------------------------------------
 // Host <-> device streaming of large arrays (particles, grids).  Caller memory
 // is ordinary pageable memory, so every copy passes through pinned staging:
-// two kPipeChunk buffers alternate, the host-side work on one chunk (a copy,
-// or the Point <-> record conversion, split over a pool of threads)
-// overlapping the DMA of the other.
+// two buffers alternate, the host-side work on one chunk (a copy, or the Point
+// <-> record conversion, split over a pool of threads) overlapping the DMA of
+// the other.
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -144,16 +144,34 @@ static int ensure_pipe(pic_ctx* c) {
     return PIC_OK;
 }
 
+// Plain copies of up to kAloneBytes go in chunks of kAloneChunk, so that the DMA
+// of one runs beside the host's copy of the other, and by the calling thread
+// alone: the pool's threads writing to fresh pages wait for each other's page
+// faults, and waking them costs more than they bring.  Larger ones go by the
+// pool.  Measured, us, pool / alone: 8.4 MB to the device 1,500 / 550, to the host
+// 1,500 / 600 (into small fresh pages 3,200 / 840); 18 MB 2,200 / 1,090 and 1,700 /
+// 1,270; 23 MB 2,600 / 1,390 and 1,900 / 1,650; 32 MB 2,900 / 1,970 and 2,000 /
+// 2,230; 36 MB to the host 2,700 / 4,100.
+constexpr size_t kAloneBytes = 24u << 20, kAloneChunk = 2u << 20;
+
+static size_t copy_chunk(size_t bytes) { return bytes <= kAloneBytes ? kAloneChunk : kPipeChunk; }
+
+static void copy_part(void* dst, const void* src, size_t m, size_t chunk) {
+    if (chunk == kAloneChunk) std::memcpy(dst, src, m);
+    else HostPool::get().copy(dst, src, m);
+}
+
 // host (pageable) -> device, enqueued on the context stream; returns when
 // the last chunk has been handed to the DMA engine.
 static int stream_to_device(pic_ctx* c, void* dev, const void* host, size_t bytes) {
     PIC_TRY(ensure_pipe(c));
     PIC_CUDA(cudaStreamSynchronize(c->stream));  // staging may still feed an earlier copy
-    for (size_t off = 0, k = 0; off < bytes; off += kPipeChunk, ++k) {
-        const size_t m = std::min(kPipeChunk, bytes - off);
+    const size_t chunk = copy_chunk(bytes);
+    for (size_t off = 0, k = 0; off < bytes; off += chunk, ++k) {
+        const size_t m = std::min(chunk, bytes - off);
         const int b = (int)(k & 1);
         if (k >= 2) PIC_CUDA(cudaEventSynchronize(c->pipe_ev[b]));  // its previous DMA is done
-        HostPool::get().copy(c->pipe_buf[b], static_cast<const char*>(host) + off, m);
+        copy_part(c->pipe_buf[b], static_cast<const char*>(host) + off, m, chunk);
         PIC_CUDA(cudaMemcpyAsync(static_cast<char*>(dev) + off, c->pipe_buf[b], m,
                                  cudaMemcpyHostToDevice, c->stream));
         PIC_CUDA(cudaEventRecord(c->pipe_ev[b], c->stream));
@@ -164,9 +182,9 @@ static int stream_to_device(pic_ctx* c, void* dev, const void* host, size_t byte
 // device -> host (pageable), after the work queued on the stream; synchronous.
 static int stream_to_host(pic_ctx* c, void* host, const void* dev, size_t bytes) {
     PIC_TRY(ensure_pipe(c));
-    const size_t nchunks = (bytes + kPipeChunk - 1) / kPipeChunk;
+    const size_t chunk = copy_chunk(bytes), nchunks = (bytes + chunk - 1) / chunk;
     auto issue = [&](size_t k) -> int {
-        const size_t off = k * kPipeChunk, m = std::min(kPipeChunk, bytes - off);
+        const size_t off = k * chunk, m = std::min(chunk, bytes - off);
         const int b = (int)(k & 1);
         PIC_CUDA(cudaMemcpyAsync(c->pipe_buf[b], static_cast<const char*>(dev) + off, m,
                                  cudaMemcpyDeviceToHost, c->stream));
@@ -180,8 +198,8 @@ static int stream_to_host(pic_ctx* c, void* host, const void* dev, size_t bytes)
         if (k + 1 < nchunks) PIC_TRY(issue(k + 1));
         const int b = (int)(k & 1);
         PIC_CUDA(cudaEventSynchronize(c->pipe_ev[b]));
-        const size_t off = k * kPipeChunk, m = std::min(kPipeChunk, bytes - off);
-        HostPool::get().copy(static_cast<char*>(host) + off, c->pipe_buf[b], m);
+        const size_t off = k * chunk, m = std::min(chunk, bytes - off);
+        copy_part(static_cast<char*>(host) + off, c->pipe_buf[b], m, chunk);
     }
     return PIC_OK;
 }

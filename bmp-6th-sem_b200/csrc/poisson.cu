@@ -1093,22 +1093,37 @@ static bool invert_level(int GX, int GY, double cx, double cy, double cd, const 
     std::vector<std::vector<int>> below(nf);  // rows k > i with L[k][i] in the envelope
     for (int k = 0; k < nf; ++k)
         for (int i = first[k]; i < k; ++i) below[i].push_back(k);
+    // kC columns at a time: each is a chain of dependent subtractions, and side by
+    // side they fill its latency (each column's operations and order are its own)
+    constexpr int kC = 8;
+    std::vector<double> LT((size_t)nf * nf);  // the factor's columns as rows
+    for (int i = 0; i < nf; ++i)
+        for (int k : below[i]) LT[(size_t)i * nf + k] = A[(size_t)k * nf + i];
     inv.assign((size_t)nf * nfp, 0.f);
-    std::vector<double> y(nf), x(nf);
-    for (int c = 0; c < nf; ++c) {
-        for (int i = 0; i < c; ++i) y[i] = 0.0;
+    std::vector<double> y((size_t)nf * kC), x((size_t)nf * kC);
+    for (int c = 0; c < nf; c += kC) {
         for (int i = c; i < nf; ++i) {
             const double* Li = &A[(size_t)i * nf];
-            double t = i == c ? 1.0 : 0.0;
-            for (int k = std::max(first[i], c); k < i; ++k) t -= Li[k] * y[k];
-            y[i] = t / Li[i];
+            double t[kC];
+            for (int q = 0; q < kC; ++q) t[q] = i == c + q ? 1.0 : 0.0;
+            for (int k = std::max(first[i], c); k < i; ++k) {
+                const double l = Li[k], *yk = &y[(size_t)k * kC];
+                for (int q = 0; q < kC; ++q) t[q] -= l * yk[q];
+            }
+            for (int q = 0; q < kC; ++q) y[(size_t)i * kC + q] = t[q] / Li[i];
         }
         for (int i = nf - 1; i >= 0; --i) {
-            double t = y[i];
-            for (int k : below[i]) t -= A[(size_t)k * nf + i] * x[k];
-            x[i] = t / A[(size_t)i * nf + i];
+            double t[kC];
+            for (int q = 0; q < kC; ++q) t[q] = i >= c ? y[(size_t)i * kC + q] : 0.0;
+            const double* LTi = &LT[(size_t)i * nf];
+            for (int k : below[i]) {
+                const double l = LTi[k], *xk = &x[(size_t)k * kC];
+                for (int q = 0; q < kC; ++q) t[q] -= l * xk[q];
+            }
+            for (int q = 0; q < kC; ++q) x[(size_t)i * kC + q] = t[q] / A[(size_t)i * nf + i];
         }
-        for (int i = 0; i < nf; ++i) inv[(size_t)i * nfp + direct_place(c)] = (float)x[i];
+        for (int i = 0; i < nf; ++i)
+            for (int q = 0; q < kC && c + q < nf; ++q) inv[(size_t)i * nfp + direct_place(c + q)] = (float)x[(size_t)i * kC + q];
     }
     return true;
 }

@@ -292,7 +292,7 @@ class Pic:
         return n.value
 
     def bin_counts(self, s: int) -> np.ndarray:
-        out = np.zeros(self.nodes, np.int32)
+        out = np.empty(self.nodes, np.int32)
         _check(lib().pic_bin_counts(self.h, s, _p(out)))
         return out
 
@@ -334,7 +334,7 @@ class Pic:
 
     # ---- grids ----
     def _grid(self, fn, *args):
-        out = np.zeros(self.nodes)
+        out = np.empty(self.nodes)
         _check(fn(self.h, *args, _p(out)))
         return out
 
@@ -351,7 +351,7 @@ class Pic:
         return self._grid(lib().pic_get_energy_mesh, s)
 
     def efield(self):
-        out = np.zeros((self.nodes, 2))
+        out = np.empty((self.nodes, 2))
         _check(lib().pic_get_efield(self.h, _p(out)))
         return out
 
