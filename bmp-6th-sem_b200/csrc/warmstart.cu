@@ -745,8 +745,11 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad_rows(const __grid_const
 // order.  Many outputs: a block takes 32 consecutive outputs, its warp w
 // sums blocks w, w + 8, ... (coalesced rows), and the eight warp sums are
 // added in order; few outputs: a warp an output, lane l summing blocks l,
-// l + 32, ..., then a fixed shuffle tree.
+// l + 32, ..., then a fixed shuffle tree.  SCATTER: outputs [tap][co][ci] (+
+// bias) go to the parameter layout [tap][ci][co] (+ bias); a kernel of its own
+// for that took 2.8 us a layer of the 390 a training step.
 constexpr int kSumWide = 256;  // outputs from which the first form is used
+template <bool SCATTER = false>
 __global__ void __launch_bounds__(256) k_sum_partials(const float* partial, int nblocks, int n, float* grad) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (n >= kSumWide) {
@@ -757,8 +760,9 @@ __global__ void __launch_bounds__(256) k_sum_partials(const float* partial, int 
             for (int b = warp; b < nblocks; b += 8) v += partial[(int64_t)b * n + i];
         red[warp][lane] = v;
         __syncthreads();
+        const int to = SCATTER && i < 9 * C * C ? (i / (C * C) * C + i % C) * C + (i / C) % C : i;
         if (warp == 0 && i < n)
-            grad[i] = ((red[0][lane] + red[1][lane]) + (red[2][lane] + red[3][lane])) +
+            grad[to] = ((red[0][lane] + red[1][lane]) + (red[2][lane] + red[3][lane])) +
                       ((red[4][lane] + red[5][lane]) + (red[6][lane] + red[7][lane]));
         return;
     }
@@ -1269,7 +1273,6 @@ struct Net {
     float* resid = nullptr;  // scaled starting residual on the node grid
     float* partial = nullptr;
     size_t partial_floats = 0;
-    float* gsum = nullptr;  // summed 32->32 weight gradient before re-layout
     float* loss_acc = nullptr;  // per-pair loss of the current epoch
     float* loss_partial = nullptr;
     // dataset of recorded pairs: x0 image (bf16, P*P*4) and target (f32, GX*GY)
@@ -1301,7 +1304,7 @@ static void net_free(Net& N) {
     for (auto* p : N.d_big) cudaFree(p);
     for (auto* p : N.d_mid) cudaFree(p);
     for (auto* p : N.d_small) cudaFree(p);
-    cudaFree(N.dout); cudaFree(N.resid); cudaFree(N.partial); cudaFree(N.loss_partial); cudaFree(N.gsum); cudaFree(N.loss_acc);
+    cudaFree(N.dout); cudaFree(N.resid); cudaFree(N.partial); cudaFree(N.loss_partial); cudaFree(N.loss_acc);
     cudaFree(N.ds_x); cudaFree(N.ds_t);
     cudaFree(N.phi_prev); cudaFree(N.b_prev); cudaFree(N.db);
     N = Net{};
@@ -1402,8 +1405,7 @@ static int ws_alloc(pic_ctx* c) {
     // per-block partials of the 32->32 weight gradients; per-row partials of
     // the outer layers'
     N.partial_floats = (size_t)std::max(kWgradBlocks, kSmallWgradBlocks) * (9 * C * C + C);
-    if (cudaMalloc(&N.partial, N.partial_floats * 4) || cudaMalloc(&N.loss_partial, g1(std::max<int64_t>(P * P, c->nodes)) * 4) ||
-        cudaMalloc(&N.gsum, (9 * C * C + C) * 4))
+    if (cudaMalloc(&N.partial, N.partial_floats * 4) || cudaMalloc(&N.loss_partial, g1(std::max<int64_t>(P * P, c->nodes)) * 4))
         return fail(PIC_ERR_CUDA, "warm start: scratch allocation failed");
     const size_t nodes = (size_t)c->nodes;
     if (cudaMalloc(&N.phi_prev, nodes * 8) || cudaMalloc(&N.b_prev, nodes * 8) ||
@@ -1560,18 +1562,6 @@ int ws_check_fault() {
     return PIC_OK;
 }
 
-// [tap][co][ci] (+ bias) -> the parameter layout [tap][ci][co] (+ bias)
-__global__ void k_scatter_wgrad(const float* src, float* g) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 9 * C * C + C) return;
-    if (i < 9 * C * C) {
-        const int tap = i / (C * C), co = (i / C) % C, ci = i % C;
-        g[(tap * C + ci) * C + co] = src[i];
-    } else {
-        g[i] = src[i];
-    }
-}
-
 // Weight gradient of 32->32 layer `layer` from its forward input (tm_wx)
 // and the gradient image tm_wd[g] of its output, on tcgen05.
 static void wgrad32(pic_ctx* c, int layer, int g, int P) {
@@ -1579,9 +1569,8 @@ static void wgrad32(pic_ctx* c, int layer, int g, int P) {
     const int units = ((P + 3) / 4) * ((P + 31) / 32);
     const int grid = std::max(1, std::min(N.sms, units));
     k_wgrad_rows<<<grid, kWgThreads, kWgSmem, c->stream>>>(N.tm_wx[layer], N.tm_wd[g], P, N.partial);
-    k_sum_partials<<<sum_blocks(9 * C * C + C), 256, 0, c->stream>>>(N.partial, grid, 9 * C * C + C,
-                                                             N.gsum);
-    k_scatter_wgrad<<<g1(9 * C * C + C), 256, 0, c->stream>>>(N.gsum, N.g + param_off(layer + 1));
+    k_sum_partials<true><<<sum_blocks(9 * C * C + C), 256, 0, c->stream>>>(N.partial, grid, 9 * C * C + C,
+                                                                           N.g + param_off(layer + 1));
 }
 
 // Forward pass on the image N.xin; result in N.out.  Thirteen launches: the
@@ -1660,7 +1649,7 @@ static void backward(pic_ctx* c) {
     conv_rows_grad(c, 0, 0, B1, P, N.a[1]);        // B1 = dPre1
     k_wgrad_in<<<kSmallWgradBlocks, 256, 0, c->stream>>>(N.xin, B1, P, N.partial);
     k_sum_partials<<<sum_blocks(kInOut), 256, 0, c->stream>>>(N.partial, kSmallWgradBlocks, kInOut, N.g);
-    c->launches += 2 + 1 + 10 * 3 + 4 + 2;
+    c->launches += 2 + 1 + 10 * 2 + 4 + 2;
 }
 
 }  // namespace picb200
