@@ -811,6 +811,9 @@ bool cluster_layout(pic_ctx* c, ClInst& I, size_t* bytes) {
         int rows = M.GY, first[kClBlocks + 1];
         L.near = kClBlocks;
         if (dist) {
+            // periodic in y: a halo of more rows than the level has would hold rows
+            // twice over, and push_rows stores a row and the two images next to it only
+            if (c->periodic && M.GY < L.H) return false;
             rows = 0;
             for (int b = 0; b <= kClBlocks; ++b) {
                 first[b] = (int)((int64_t)b * ps.levels[0].GY / kClBlocks);
