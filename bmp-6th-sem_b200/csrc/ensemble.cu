@@ -50,7 +50,7 @@ struct pic_ensemble {
     bool energy = true;
     bool use_graph = true;
     cudaGraphExec_t graph = nullptr;
-    int graph_kernels = 0;  // batch_kernels() of the captured step
+    int64_t graph_kernels = 0;  // batch_kernels() of the captured step
     bool graph_failed = false;
     double last_ms[3] = {0, 0, 0};  // deposit, Poisson (+E), push
 };
@@ -255,7 +255,7 @@ int pic_ensemble_step(pic_ensemble* e, int iteration) {
             if (!c->sp[s].acc_fresh) PIC_TRY(particles_deposit(c, s));
     PIC_TRY(batch_prepare(e->pb, e->cs.data(), e->stream));
     PIC_TRY(upload_poisson(e));
-    const int kernels = batch_kernels(e->pb, e->shape);
+    const int64_t kernels = batch_kernels(e->pb, e->shape);
     if (e->graph && e->graph_kernels != kernels) {
         PIC_CUDA(cudaGraphExecDestroy(e->graph));  // captured with other push kernels
         e->graph = nullptr;

@@ -1376,7 +1376,7 @@ int pick_lanes(double ppc) { return ppc >= 48.0 ? 16 : (ppc >= 12.0 ? 8 : 4); }
 struct CellLaunch {
     int tile;   // index into kTile
     int lanes;  // lanes a cell of a push
-    bool bzu;   // uniform Bz (in every instance)
+    bool bzu;   // uniform Bz
 };
 
 CellLaunch cell_launch(const pic_ctx* c, const Species& sp) {
@@ -2051,8 +2051,12 @@ __global__ void __launch_bounds__(256) k_fixup_batch(const FixArgs* __restrict__
 
 struct ParticleBatchImpl {
     int n = 0, ns = 0;
+    // each tile shape's {instance, tile} of every block: the instances whose Bz is
+    // uniform first, the others from block nuniform on
     uint2* work[kNumTiles] = {};
-    unsigned nblocks[kNumTiles] = {};
+    unsigned nblocks[kNumTiles] = {}, nuniform[kNumTiles] = {};
+    std::vector<bool> uniform;  // each instance's Bz when the lists were made
+    int64_t lists_made = 0;
     KArgs* d_args = nullptr;      // [ns][n] pushes, then [ns][n] deposits of arrivals
     FixArgs* d_fix = nullptr;     // [ns][n]
     FlushEntry* d_flush = nullptr;  // [ns][n]
@@ -2064,10 +2068,35 @@ struct ParticleBatchImpl {
     unsigned long long* h_flags = nullptr;  // pinned, [ns][n]: push_report() of each push
     int64_t max_nodes = 0;  // nodes of the largest instance
     double ppc = 0;         // particles a cell, over all instances and species
-    bool bzu = true;        // every instance's Bz is uniform
 };
 
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+// Makes the work lists, unless every instance's Bz is of the kind that it was
+// when they were made.  (Their lengths do not change.)
+static int batch_work(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st) {
+    std::vector<bool> uniform;
+    for (int i = 0; i < B->n; ++i) uniform.push_back(cs[i]->bz_uniform);
+    if (B->lists_made && uniform == B->uniform) return PIC_OK;
+    for (int sh = 0; sh < kNumTiles; ++sh) {
+        std::vector<uint2> w;
+        for (const bool kind : {true, false}) {
+            for (int i = 0; i < B->n; ++i) {
+                if (uniform[i] != kind) continue;
+                const unsigned tiles = num_tiles(cs[i], kTile[sh]);
+                for (unsigned t = 0; t < tiles; ++t) w.push_back(make_uint2((uint32_t)i, t));
+            }
+            if (kind) B->nuniform[sh] = (unsigned)w.size();
+        }
+        B->nblocks[sh] = (unsigned)w.size();
+        if (!B->work[sh]) PIC_CUDA(cudaMalloc(&B->work[sh], w.size() * sizeof(uint2)));
+        PIC_CUDA(cudaMemcpyAsync(B->work[sh], w.data(), w.size() * sizeof(uint2), cudaMemcpyHostToDevice, st));
+    }
+    PIC_CUDA(cudaStreamSynchronize(st));
+    B->uniform = uniform;
+    B->lists_made += 1;
+    return PIC_OK;
+}
 
 int batch_create(pic_ctx** cs, int n, ParticleBatchImpl** out) {
     auto* B = new ParticleBatchImpl();
@@ -2075,16 +2104,7 @@ int batch_create(pic_ctx** cs, int n, ParticleBatchImpl** out) {
     B->n = n;
     B->ns = cs[0]->cfg.num_species;
     for (int i = 0; i < n; ++i) B->max_nodes = std::max<int64_t>(B->max_nodes, cs[i]->nodes);
-    for (int sh = 0; sh < kNumTiles; ++sh) {
-        std::vector<uint2> w;
-        for (int i = 0; i < n; ++i) {
-            const unsigned tiles = num_tiles(cs[i], kTile[sh]);
-            for (unsigned t = 0; t < tiles; ++t) w.push_back(make_uint2((uint32_t)i, t));
-        }
-        B->nblocks[sh] = (unsigned)w.size();
-        PIC_CUDA(cudaMalloc(&B->work[sh], w.size() * sizeof(uint2)));
-        PIC_CUDA(cudaMemcpy(B->work[sh], w.data(), w.size() * sizeof(uint2), cudaMemcpyHostToDevice));
-    }
+    PIC_TRY(batch_work(B, cs, cs[0]->stream));
     const int ns = B->ns;
     size_t off = 0;
     auto carve = [&](size_t bytes) {
@@ -2138,11 +2158,10 @@ int batch_prepare(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st) {
     FixArgs* hf = reinterpret_cast<FixArgs*>(B->h_tables + o_fix);
     FlushEntry* hl = reinterpret_cast<FlushEntry*>(B->h_tables + o_flush);
     ZeroEntry* hz = reinterpret_cast<ZeroEntry*>(B->h_tables + o_zero);
-    B->bzu = true;
+    PIC_TRY(batch_work(B, cs, st));
     double cells = 0, count = 0;
     for (int i = 0; i < n; ++i) {
         pic_ctx* c = cs[i];
-        B->bzu = B->bzu && c->bz_uniform;
         for (int s = 0; s < ns; ++s) {
             cells += (double)c->ncells;
             count += (double)c->ncells * c->sp[s].ppc;
@@ -2166,14 +2185,27 @@ int batch_prepare(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st) {
 }
 
 static CellLaunch batch_launch(const ParticleBatchImpl* B, int shape) {
-    return CellLaunch{pick_tile(shape, B->ppc, B->nblocks[4]), pick_lanes(B->ppc), B->bzu};
+    return CellLaunch{pick_tile(shape, B->ppc, B->nblocks[4]), pick_lanes(B->ppc), true};
 }
 
 // The kernels that a push of the batch launches, as a number: a captured
 // step is good for as long as it does not change.
-int batch_kernels(const ParticleBatchImpl* B, int shape) {
+int64_t batch_kernels(const ParticleBatchImpl* B, int shape) {
     const CellLaunch L = batch_launch(B, shape);
-    return (L.tile * 64 + L.lanes) * 2 + (L.bzu ? 1 : 0);
+    return (B->lists_made * kNumTiles + L.tile) * 64 + L.lanes;
+}
+
+// The push pass of species s of every instance: one launch for the instances
+// whose Bz is uniform, one for the others.  (An instance's push is then the one
+// that it has in a context of its own, whatever the others' Bz.)
+template <bool ENERGY>
+static void launch_push_batch(const ParticleBatchImpl* B, CellLaunch L, int s, cudaStream_t st) {
+    const unsigned nu = B->nuniform[L.tile], nv = B->nblocks[L.tile] - nu;
+    const KArgs* args = B->d_args + (size_t)s * B->n;
+    L.bzu = true;
+    if (nu) launch_cells_batch<kPush, ENERGY>(L, nu, st, args, B->work[L.tile]);
+    L.bzu = false;
+    if (nv) launch_cells_batch<kPush, ENERGY>(L, nv, st, args, B->work[L.tile] + nu);
 }
 
 // Flush the accumulators of every species of every instance into final/energy
@@ -2191,10 +2223,8 @@ int batch_push(ParticleBatchImpl* B, int shape, bool energy, cudaStream_t st) {
     const int n = B->n, ns = B->ns;
     const CellLaunch cl = batch_launch(B, shape);
     for (int s = 0; s < ns; ++s) {
-        if (energy)
-            launch_cells_batch<kPush, true>(cl, B->nblocks[cl.tile], st, B->d_args + (size_t)s * n, B->work[cl.tile]);
-        else
-            launch_cells_batch<kPush, false>(cl, B->nblocks[cl.tile], st, B->d_args + (size_t)s * n, B->work[cl.tile]);
+        if (energy) launch_push_batch<true>(B, cl, s, st);
+        else launch_push_batch<false>(B, cl, s, st);
         if (energy)
             launch_cells_batch<kArrivals, true>(cl, B->nblocks[cl.tile], st, B->d_args + (size_t)(ns + s) * n, B->work[cl.tile]);
         else
@@ -2249,10 +2279,8 @@ int batch_time_shapes(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st, int r
             cudaEventRecord(e0, st);
             for (int s = 0; s < ns; ++s) {
                 k_batch_zero<<<296, 256, 0, st>>>(B->d_zero + (size_t)s * 2 * n, 2 * n);
-                if (energy)
-                    launch_cells_batch<kPush, true>(cl, B->nblocks[cl.tile], st, B->d_args + (size_t)s * n, B->work[cl.tile]);
-                else
-                    launch_cells_batch<kPush, false>(cl, B->nblocks[cl.tile], st, B->d_args + (size_t)s * n, B->work[cl.tile]);
+                if (energy) launch_push_batch<true>(B, cl, s, st);
+                else launch_push_batch<false>(B, cl, s, st);
             }
             cudaEventRecord(e1, st);
             if (cudaEventSynchronize(e1) != cudaSuccess || cudaGetLastError() != cudaSuccess) {

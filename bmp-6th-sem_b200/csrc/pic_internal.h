@@ -313,7 +313,7 @@ int batch_create(pic_ctx** cs, int n, ParticleBatchImpl** out);
 void batch_destroy(ParticleBatchImpl* B);
 int batch_prepare(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st);
 int batch_deposit(ParticleBatchImpl* B, cudaStream_t st);
-int batch_kernels(const ParticleBatchImpl* B, int shape);
+int64_t batch_kernels(const ParticleBatchImpl* B, int shape);
 int batch_push(ParticleBatchImpl* B, int shape, bool energy, cudaStream_t st);
 void batch_commit(pic_ctx** cs, int n);
 int batch_time_shapes(ParticleBatchImpl* B, pic_ctx** cs, cudaStream_t st, int reps, bool energy,
