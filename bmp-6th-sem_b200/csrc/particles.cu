@@ -97,13 +97,16 @@ struct KArgs {
     int64_t ncells;
     SpeciesConsts k;
     const float4* __restrict__ fld;
-    const float4* __restrict__ src_a;
-    const float* __restrict__ src_vz;
+    // (not __restrict__, like back_src: the arrivals' pass reads what the kernel
+    // before it wrote, and may be launched before that one's end; its loads must
+    // stay behind the wait)
+    const float4* src_a;
+    const float* src_vz;
     float4* __restrict__ dst_a;
     float* __restrict__ dst_vz;
     const uint32_t* __restrict__ base;
     const uint32_t* __restrict__ front_src;
-    const uint32_t* __restrict__ back_src;
+    const uint32_t* back_src;
     uint32_t* front_dst;
     uint32_t* back_dst;
     ListDev ovf;
@@ -782,7 +785,7 @@ struct FixArgs {
     float4* dst_a;
     float* dst_vz;
     const uint32_t* __restrict__ base;
-    const uint32_t* __restrict__ front;  // final front counts of the new buffer
+    const uint32_t* front;  // final front counts of the new buffer
     uint32_t* back;                      // back counts of the new buffer
     ListDev ovf;    // pushed this step, not yet placed
     ListDev prev;   // part of the state before the push, not yet pushed

@@ -1129,10 +1129,12 @@ static bool invert_level(int GX, int GY, double cx, double cy, double cd, const 
 }
 
 // x[free_idx[i]] = sum_j inv[i][j] b[free_idx[j]]: a warp a row (lanes over
-// j, then a fixed shuffle tree), b's free values staged in shared memory.  The first groups of the row are loaded before the wait for
-// the kernel before (the inverse does not change).
+// j, then a fixed shuffle tree), b's free values staged in shared memory.  The
+// first groups of the row are loaded before the wait for the kernel before (the
+// inverse does not change; b, which that kernel writes, is not __restrict__: its
+// loads must stay behind the wait).
 __global__ void __launch_bounds__(256) k_mg_direct(const float* __restrict__ inv, const int* __restrict__ freen,
-                                                   int nf, int nfp, const float* __restrict__ b, float* __restrict__ x) {
+                                                   int nf, int nfp, const float* b, float* x) {
     extern __shared__ float4 bs4[];
     float* bs = reinterpret_cast<float*>(bs4);
     const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5), n4 = nfp / 4;
@@ -2073,7 +2075,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_poisson_batch(const BatchInst
     const int group = (blockIdx.x - I->blk0) * (NT / kTileThreads) + grp, groups = I->nblk * (NT / kTileThreads);
     TileMem& T = reinterpret_cast<TileMem*>(smem)[grp];
     const uint8_t* __restrict__ mk = I->mask;
-    const float* __restrict__ z = kf > 0 ? I->xo[0] : I->lev[0].x;
+    const float* z_of = kf > 0 ? I->xo[0] : I->lev[0].x;  // what the V-cycle writes in every iteration
     const int nn = (int)I->sn, GX = I->GX;
     const double cd = I->cd, cx = I->cx, cy = I->cy;
     // the summing blocks' threads and warps; the first of this warp's, spread over the blocks
@@ -2113,6 +2115,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_poisson_batch(const BatchInst
         for (int vw = vw0; vw < vws; vw += vwn) {
             double a = 0.0;
             const double* __restrict__ rv = I->r;
+            const float* __restrict__ z = z_of;  // (only read in this pass, as in the next)
             for (int k0 = 32 * vw + lane; k0 < nn; k0 += 8 * vsize) {
                 double r[8];
                 float zk[8];
@@ -2138,6 +2141,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_poisson_batch(const BatchInst
         const double beta = rz_old == 0.0 ? 0.0 : rz / rz_old;
         for (int vw = vw0; vw < vws; vw += vwn) {
             double a = 0.0;
+            const float* __restrict__ z = z_of;
             const double* __restrict__ po = I->p[it & 1];
             double* __restrict__ pv = I->p[(it & 1) ^ 1];
             double* __restrict__ qv = I->q;
