@@ -470,7 +470,7 @@ constexpr int kTileNodes = 2 * (kTileCells + 1);  // of the widest tile, 256 x 1
 // of 2, and with 8 blocks of 4 warps at 64 registers, the push of the 1024^2
 // workload took 3 to 8 % longer.
 constexpr int kCellBlocksPerSM = 6;
-constexpr int kDepth = 3;  // chunks in the ring  // chunks in the ring
+constexpr int kDepth = 3;  // chunks in the ring
 
 struct Tile {
     int ltx, lty;  // log2 of the cells in x and y
@@ -546,47 +546,55 @@ __device__ __forceinline__ uint32_t place_movers(const KArgs& A, MoverQueue& q,
     return left;
 }
 
+template <int MODE, bool BZU>
+struct CellShared {
+    CellMeta meta[kTileCells];
+    NodeField<BZU> fld[MODE == kPush ? kTileNodes : 1];
+    MoverQueue q[MODE == kPush ? kWarps : 1];
+    float4 ring_a[kWarps][kDepth][2][32];
+    float ring_vz[kWarps][kDepth][2][32];
+};
+
+// Whether the warps of a block would be done clearly sooner with all 32 lanes on
+// a cell than with G, by the particle counts n of 32 neighbouring cells, one a
+// lane: G lanes a set of 32 / G cells take as many chunks as the set's fullest
+// cell needs, so a cell far fuller than its neighbours (a beam spot, a sheath) is
+// walked 2 G particles at a time by one warp while the others are done.
+// Measured, us a push of Ar+, 256^2 cells, 2 a cell and one of 2,000 / 8,000 /
+// 40,000: 4 lanes throughout 119 / 412 / 1,974, with this 39 / 73 / 255; 512^2, 4 a
+// cell and a blob of 20,000 a cell at its centre, sigma 3 cells: 990 / 205.  Where
+// no tile is crowded the look at the counts costs 0.4 % (1024^2 workload, both
+// species 2,138 / 2,148 us) to 1 % (512^2, 369 / 373).
+template <int G>
+__device__ __forceinline__ bool crowded(uint32_t n) {
+    // (evenly filled cells, which is nearly all: nothing more to do)
+    if (__reduce_max_sync(kFull, n) <= (__reduce_add_sync(kFull, n) >> 5) + 64u) return false;
+    constexpr int kSetCells = 32 / G;
+    uint32_t narrow = n;  // the fullest of the lane's set
+#pragma unroll
+    for (int d = 1; d < kSetCells; d <<= 1) narrow = max(narrow, __shfl_xor_sync(kFull, narrow, d));
+    narrow = (narrow + 2 * G - 1) / (2 * G);
+    // the sets, and the cells, that go to one warp
+#pragma unroll
+    for (int d = kWarps * kSetCells; d < 32; d <<= 1) narrow += __shfl_xor_sync(kFull, narrow, d);
+    uint32_t wide = (n + 63) / 64;
+#pragma unroll
+    for (int d = kWarps; d < 32; d <<= 1) wide += __shfl_xor_sync(kFull, wide, d);
+    return 4 * __reduce_max_sync(kFull, wide) <= 3 * __reduce_max_sync(kFull, narrow);
+}
+
+// The tile's cells, G lanes a cell (its metadata and fields are in S).
 template <int MODE, bool ENERGY, bool BZU, int G>
-__device__ __forceinline__ void cells_body(const KArgs& A, Tile T, uint32_t tile) {
+__device__ __forceinline__ void cells_run(const KArgs& A, Tile T, int tgx0, int tgy0, CellShared<MODE, BZU>& S) {
     constexpr int kSetCells = 32 / G;  // cells a warp works on at a time (neighbours in a row)
-    __shared__ CellMeta s_meta[kTileCells];
     using Field = NodeField<BZU>;
-    __shared__ Field s_fld[MODE == kPush ? kTileNodes : 1];
-    __shared__ MoverQueue s_q[MODE == kPush ? kWarps : 1];
-    __shared__ float4 s_ring_a[kWarps][kDepth][2][32];
-    __shared__ float s_ring_vz[kWarps][kDepth][2][32];
+    const CellMeta* s_meta = S.meta;
+    const Field* s_fld = S.fld;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gl = lane & (G - 1), grp = lane / G;  // lane of the group, group of the warp
-    const int cells = 1 << (T.ltx + T.lty), sets = cells / kSetCells;
-    // tiles in row order: the blocks resident at a time work on one stretch
-    // of the slot arrays
-    const uint32_t tiles_x = (uint32_t)(A.nx + (1 << T.ltx) - 1) >> T.ltx, tile_y = tile / tiles_x;
-    const int tgx0 = (int)(tile - tile_y * tiles_x) << T.ltx, tgy0 = (int)tile_y << T.lty;
+    const int sets = (1 << (T.ltx + T.lty)) / kSetCells, rowlen = (1 << T.ltx) + 1;
     const unsigned lt = lanemask_lt();
     const unsigned gmask = (G == 32 ? kFull : ((1u << (G & 31)) - 1u)) << (grp * G);
-    for (int i = threadIdx.x; i < cells; i += kThreads) {
-        const int gx = tgx0 + (i & ((1 << T.ltx) - 1)), gy = tgy0 + (i >> T.ltx);
-        CellMeta m{0u, 0u, 0u, 0u};
-        if (gx < A.nx && gy < A.ny) {
-            const int64_t c = (int64_t)gy * A.nx + gx;
-            m.b0 = A.base[c];
-            m.b1 = A.base[c + 1];
-            m.nf = MODE == kArrivals ? 0u : A.front_src[c];
-            m.nb = A.back_src[c];
-        }
-        s_meta[i] = m;
-    }
-    const int rowlen = (1 << T.ltx) + 1;
-    if (MODE == kPush) {
-        const int nodes = rowlen * ((1 << T.lty) + 1);
-        for (int i = threadIdx.x; i < nodes; i += kThreads) {
-            const int ly = i / rowlen, x = tgx0 + (i - ly * rowlen), y = tgy0 + ly;
-            s_fld[i] = Field::from((x < A.GX && y < A.ny + 1) ? __ldg(A.fld + (int64_t)y * A.GX + x)
-                                                              : make_float4(0.f, 0.f, 0.f, 0.f));
-        }
-    }
-    __syncthreads();
-
     uint32_t left_exits = 0;  // per lane
     // The set being loaded: the group's cell as the source index of its j-th
     // particle (the front run for j < pnf, then the back run, index pback +
@@ -607,8 +615,8 @@ __device__ __forceinline__ void cells_body(const KArgs& A, Tile T, uint32_t tile
         }
         pj = gl;
     };
-    const uint32_t ring_a0 = smem_u32(&s_ring_a[warp][0][0][lane]);
-    const uint32_t ring_vz0 = smem_u32(&s_ring_vz[warp][0][0][lane]);
+    const uint32_t ring_a0 = smem_u32(&S.ring_a[warp][0][0][lane]);
+    const uint32_t ring_vz0 = smem_u32(&S.ring_vz[warp][0][0][lane]);
     // issues the copies of the next chunk into ring slot r; every call
     // commits one (possibly empty) copy group
     auto fetch = [&](uint32_t r) {
@@ -632,7 +640,7 @@ __device__ __forceinline__ void cells_body(const KArgs& A, Tile T, uint32_t tile
     };
     p_enter();
 
-    MoverQueue& q = s_q[MODE == kPush ? warp : 0];
+    MoverQueue& q = S.q[MODE == kPush ? warp : 0];
     int queued = 0;  // warp-uniform
     // the set being worked on: the group's cell (index lc in the tile), its
     // particle count n, its corner in the shared fields, its lower left node
@@ -681,8 +689,8 @@ __device__ __forceinline__ void cells_body(const KArgs& A, Tile T, uint32_t tile
             }
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                const float4 a = s_ring_a[warp][r][u][lane];
-                vz[u] = s_ring_vz[warp][r][u][lane];
+                const float4 a = S.ring_a[warp][r][u][lane];
+                vz[u] = S.ring_vz[warp][r][u][lane];
                 const bool valid = j0 + gl + u * G < n;
                 if (MODE != kPush) {
                     p[u].fx = a.x; p[u].fy = a.y; p[u].vx = a.z; p[u].vy = a.w;
@@ -747,6 +755,41 @@ __device__ __forceinline__ void cells_body(const KArgs& A, Tile T, uint32_t tile
         const uint32_t left = __reduce_add_sync(kFull, left_exits);
         if (lane == 0 && left) atomicAdd(A.counters, (unsigned long long)left);
     }
+}
+
+template <int MODE, bool ENERGY, bool BZU, int G>
+__device__ __forceinline__ void cells_body(const KArgs& A, Tile T, uint32_t tile) {
+    __shared__ CellShared<MODE, BZU> S;
+    const int cells = 1 << (T.ltx + T.lty);  // (a multiple of 32: whole warps below)
+    // tiles in row order: the blocks resident at a time work on one stretch
+    // of the slot arrays
+    const uint32_t tiles_x = (uint32_t)(A.nx + (1 << T.ltx) - 1) >> T.ltx, tile_y = tile / tiles_x;
+    const int tgx0 = (int)(tile - tile_y * tiles_x) << T.ltx, tgy0 = (int)tile_y << T.lty;
+    bool wide = false;
+    for (int i = threadIdx.x; i < cells; i += kThreads) {
+        const int gx = tgx0 + (i & ((1 << T.ltx) - 1)), gy = tgy0 + (i >> T.ltx);
+        CellMeta m{0u, 0u, 0u, 0u};
+        if (gx < A.nx && gy < A.ny) {
+            const int64_t c = (int64_t)gy * A.nx + gx;
+            m.b0 = A.base[c];
+            m.b1 = A.base[c + 1];
+            m.nf = MODE == kArrivals ? 0u : A.front_src[c];
+            m.nb = A.back_src[c];
+        }
+        S.meta[i] = m;
+        wide = wide || crowded<G>(m.nf + m.nb);
+    }
+    const int rowlen = (1 << T.ltx) + 1;
+    if (MODE == kPush) {
+        const int nodes = rowlen * ((1 << T.lty) + 1);
+        for (int i = threadIdx.x; i < nodes; i += kThreads) {
+            const int ly = i / rowlen, x = tgx0 + (i - ly * rowlen), y = tgy0 + ly;
+            S.fld[i] = NodeField<BZU>::from((x < A.GX && y < A.ny + 1) ? __ldg(A.fld + (int64_t)y * A.GX + x)
+                                                                       : make_float4(0.f, 0.f, 0.f, 0.f));
+        }
+    }
+    if (__syncthreads_or(wide)) cells_run<MODE, ENERGY, BZU, 32>(A, T, tgx0, tgy0, S);
+    else cells_run<MODE, ENERGY, BZU, G>(A, T, tgx0, tgy0, S);
 }
 
 // The tiles of the tile shapes 1, 2 and 3 (256 cells), and the two that shape
