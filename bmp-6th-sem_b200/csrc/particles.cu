@@ -946,11 +946,13 @@ __global__ void __launch_bounds__(256) k_list_deposit(ListDev L, int nx, int GX,
 //
 // Slot capacity of a cell holding n particles: n + n/2 + 16 (room for a
 // step's incoming movers and for the count to drift between re-layouts),
-// rounded up to a multiple of 8 so that every cell's run starts on a 128-byte
+// rounded down to a multiple of 8 so that every cell's run starts on a 128-byte
 // line of the float4 array and a 32-byte sector of vz (unaligned runs took
 // the Ar+ push of the 1024^2 workload from 0.93 to 1.03 ms: more lines and
-// sectors an access).
-__host__ __device__ __forceinline__ uint32_t cell_capacity(uint32_t n) { return (n + n / 2u + 23u) & ~7u; }
+// sectors an access).  Down, not up: 24 slots for a cell of one particle in
+// place of 16 or 17 took two fifths more memory, and grids that had fitted the
+// device or the 32-bit slot indices no longer did.
+__host__ __device__ __forceinline__ uint32_t cell_capacity(uint32_t n) { return (n + n / 2u + 16u) & ~7u; }
 
 // cnt[c] = front[c] + back[c]
 __global__ void k_cell_counts(const uint32_t* front, const uint32_t* back, int64_t ncells, uint32_t* cnt) {
@@ -991,7 +993,7 @@ __global__ void __launch_bounds__(256) k_scan_partials(const uint32_t* in, int64
 }
 
 // out[t] = sum of values before t, out[n] = total.  With CAP the values are
-// cell capacities, and cells above kMaxPerCell raise counters[1].
+// cell capacities, and cells that want more than kMaxPerCell raise counters[1].
 template <bool CAP>
 __global__ void __launch_bounds__(256) k_scan_apply(const uint32_t* in, int64_t n,
                                                     const uint32_t* partials, uint32_t* out,
@@ -1012,9 +1014,10 @@ __global__ void __launch_bounds__(256) k_scan_apply(const uint32_t* in, int64_t 
     uint32_t tsum = 0, vmax = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        v[j] = (c0 + j < n) ? scan_value<CAP>(in, c0 + j) : 0u;
+        const uint32_t count = (c0 + j < n) ? in[c0 + j] : 0u;
+        v[j] = !CAP ? count : (c0 + j < n ? cell_capacity(count) : 0u);
         tsum += v[j];
-        vmax = max(vmax, v[j]);
+        vmax = max(vmax, count);
     }
     uint32_t incl = tsum;
 #pragma unroll
@@ -1034,7 +1037,7 @@ __global__ void __launch_bounds__(256) k_scan_apply(const uint32_t* in, int64_t 
         run += v[j];
         if (t == n - 1) out[n] = run;
     }
-    if (CAP && vmax > kMaxPerCell) atomicOr(counters + 1, 1ull);
+    if (CAP && vmax + vmax / 2u + 16u > kMaxPerCell) atomicOr(counters + 1, 1ull);
 }
 
 // Copies every cell's particles (front run, then back run) from the old
@@ -1657,7 +1660,7 @@ int check_flags(pic_ctx* c, Species& sp, bool sync) {
 
 // Particles a cell, on average, of a layout of `slots` slots (cell_capacity).
 static double mean_count(const pic_ctx* c, uint32_t slots) {
-    return std::max(0.0, ((double)slots / (double)c->ncells - 19.5) / 1.5);
+    return std::max(0.0, ((double)slots / (double)c->ncells - 12.5) / 1.5);
 }
 
 // Rebuilds the layout from the current per-cell counts (cell runs plus the
