@@ -41,6 +41,13 @@ constexpr int kClBlocks = 16;      // a cluster (non-portable size)
 // 276 / 250; us a step of a run (host work included): 33^2 83 / 113, 65^2 160 /
 // 190, 97^2 204 / 223, 113^2 213 / 222, 129^2 226 / 222.
 constexpr int64_t kClMaxNodes = 14000;
+// And up to this many rows of level 0 (40 a block: every one of them is walked in
+// push_rows, and narrow rows are padded).  Measured, us a solve, cluster / kernels /
+// the kernels before their tiles held quads: periodic 7 x 480 cells 185 / 193 / 230,
+// 16 x 640 251 / 220 / 266, 7 x 800 221 / 190 / 221, 7 x 1600 286 / 193 / 229, 10 x 1200
+// 309 / 223 / 268; walls 8 x 480 310 / 310 / 336, 12 x 640 222 / 215 / 267, 8 x 1200 255 /
+// 218 / 259.
+constexpr int kClMaxRows = 641;
 constexpr int kClThreads = 1024;
 constexpr int kClMaxLevels = 8;
 constexpr int kClRepNodes = 1500;  // levels up to this size are replicated
@@ -777,7 +784,7 @@ constexpr size_t kClMaxSmem = 227 * 1024 - 4096;  // dynamic; the rest is static
 bool cluster_layout(pic_ctx* c, ClInst& I, size_t* bytes) {
     PoissonState& ps = c->ps;
     const int kf = ps.fused_first;
-    if (!ps.mg_ok || kf > kClMaxLevels || c->nodes > kClMaxNodes) return false;
+    if (!ps.mg_ok || kf > kClMaxLevels || c->nodes > kClMaxNodes || ps.levels[0].GY > kClMaxRows) return false;
     size_t off = 0;
     auto carve = [&](size_t b) {
         const size_t o = off;

@@ -39,9 +39,11 @@ def _solve(pic, k, rho):
     # periodic, two distributed levels
     (100, 96, True, False, True), (60, 192, True, True, True), (180, 64, True, True, True), (90, 144, True, False, True),
     # walls: long and narrow (bands of no row; of 1,000 columns the halos do not fit the
-    # shared memory), tall and narrow, the largest and one too large
+    # shared memory), too many rows, the largest and one too large
     (300, 12, False, False, True), (600, 12, False, False, True), (1000, 12, False, False, False),
-    (14, 900, False, False, True), (500, 16, False, True, True),
+    (14, 900, False, False, False), (500, 16, False, True, True),
+    # the most rows, and one more
+    (20, 640, False, False, True), (20, 641, False, False, False), (19, 640, True, False, True), (7, 1600, True, False, False),
     (117, 117, False, True, True), (118, 118, False, True, False),
 ])
 def test_solver_and_halo_rows(nx, ny, periodic, inner, cluster):
