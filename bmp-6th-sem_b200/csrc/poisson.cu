@@ -1874,7 +1874,7 @@ namespace picb200 {
 namespace {
 
 constexpr int kMaxBatchLevels = 10;
-constexpr int kMaxSumBlocks = 512;  // (an SM a block)
+constexpr int kMaxSumBlocks = 512;  // of an instance: those that sum, those that work
 // Threads of the batch's blocks: 1,024, one block an SM, or 512, two of them.
 // With half-SM blocks the instances' shares come out more even, and one block
 // works while the other waits at a barrier; with whole ones the barriers have
@@ -1882,10 +1882,11 @@ constexpr int kMaxSumBlocks = 512;  // (an SM a block)
 // threads.
 constexpr int kBatchWhole = 1024, kBatchHalf = 512;
 // Half ones from this many nodes an SM (measured, ms a solve, whole / half:
-// 64 instances of 128^2 .. 384^2 cells, 29,000 nodes an SM, 4.22 / 3.55; 100 of
-// 64^2 .. 256^2, 21,000, 2.53 / 2.31; 24 of 128^2 .. 384^2, 11,000, 2.15 / 1.83;
-// 16 of 256^2 .. 384^2, 11,000, 1.92 / 1.92; 140 of 64^2 .. 128^2, 9,000, 1.19 /
-// 1.21; 3 of 500^2 .. 700^2, 7,000, 1.82 / 1.93; 16 of 64^2 .. 128^2, 0.66 / 0.77).
+// 64 instances of 128^2 .. 384^2 cells, 28,700 to 32,700 nodes an SM, 3.26 / 2.93,
+// 3.91 / 3.54, 3.75 / 3.48, 4.19 / 3.75 and, the one set where it loses, 3.30 /
+// 3.59; 100 of 64^2 .. 256^2, 18,300, 2.62 / 2.20; 24 of 128^2 .. 384^2, 10,100, 1.82 /
+// 1.70; 16 of 256^2 .. 384^2, 10,800, 1.76 / 1.75; 40 of 128^2 .. 256^2, 9,950, 1.49 /
+// 1.56; 8 of 256^2 .. 384^2, 5,700, 1.40 / 1.51; 16 of 64^2 .. 128^2, 0.68 / 0.84).
 constexpr int64_t kBatchHalfNodes = 10000;
 constexpr int kSumWarps = 32;  // of a summing block
 
@@ -1970,7 +1971,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_poisson_batch(const BatchInst
                                                                   int* err) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double s_red[2][NT / 32];
-    __shared__ double s_total;
     __shared__ double s_blk[kMaxSumBlocks];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int me = inst_of[blockIdx.x];  // -1: a spare block
@@ -1995,16 +1995,14 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_poisson_batch(const BatchInst
             partials[2 * blockIdx.x + slot] = t;
         }
     };
-    // after a barrier: the sum over the instance's blocks, fixed order
+    // after a barrier: the sum over the instance's blocks, fixed order (all loads in
+    // one round trip, as below)
     auto total = [&](int slot) {
-        if (threadIdx.x == 0) {
-            double t = 0.0;
-#pragma unroll 4
-            for (int b = I->blk0; b < I->blk0 + I->nblk; ++b) t += __ldcg(partials + 2 * b + slot);
-            s_total = t;
-        }
+        const int nb = I->nblk;
+        for (int b = threadIdx.x; b < nb; b += NT) s_blk[b] = __ldcg(partials + 2 * (I->blk0 + b) + slot);
         __syncthreads();
-        const double t = s_total;
+        double t = 0.0;
+        for (int b = 0; b < nb; ++b) t += s_blk[b];
         __syncthreads();
         return t;
     };
@@ -2014,14 +2012,21 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_poisson_batch(const BatchInst
         for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
         if (lane == 0) I->wsum[slot * I->sumblk * kSumWarps + vw] = a;
     };
-    // after a barrier: the summing blocks' warps in order, then those blocks in order
+    // after a barrier: the summing blocks' warps in order, then those blocks in
+    // order; of the warps only those that have a node (the others' sums are 0).
+    // All loads in one round trip, through the tiles' shared memory.  With loads in
+    // turn, of the empty warps' too, a solve of 1 instance of 16^2 cells took 461 us, of
+    // 3 of them 295, of 100 of 64^2 432, of 1 of 900^2 2,090; with this 221, 209, 407, 1,689.
+    const int sum_warps = min(I->sumblk * kSumWarps, ((int)I->sn + 31) / 32);
     auto ordered_total = [&](int slot) {
-        const int sb = I->sumblk;
+        const int sb = (sum_warps + kSumWarps - 1) / kSumWarps;
+        double* sw = reinterpret_cast<double*>(smem);  // (rows of 33: no bank conflicts)
+        const double* w = I->wsum + (int64_t)slot * I->sumblk * kSumWarps;
+        for (int n = threadIdx.x; n < sum_warps; n += NT) sw[(n >> 5) * (kSumWarps + 1) + (n & 31)] = __ldcg(w + n);
+        __syncthreads();
         for (int b = threadIdx.x; b < sb; b += NT) {
-            const double* w = I->wsum + ((int64_t)slot * sb + b) * kSumWarps;
             double t = 0.0;
-#pragma unroll 8
-            for (int n = 0; n < kSumWarps; ++n) t += __ldcg(w + n);
+            for (int n = 0; n < min(kSumWarps, sum_warps - b * kSumWarps); ++n) t += sw[b * (kSumWarps + 1) + n];
             s_blk[b] = t;
         }
         __syncthreads();
@@ -2079,7 +2084,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_poisson_batch(const BatchInst
     const int nn = (int)I->sn, GX = I->GX;
     const double cd = I->cd, cx = I->cx, cy = I->cy;
     // the summing blocks' threads and warps; the first of this warp's, spread over the blocks
-    const int vws = I->sumblk * kSumWarps, vsize = 32 * vws, vwn = I->nblk * (NT / 32);
+    const int vws = sum_warps, vsize = 32 * I->sumblk * kSumWarps, vwn = I->nblk * (NT / 32);
     const int vw0 = (int)(blockIdx.x - I->blk0) + I->nblk * warp;
     while (go) {
         // ---- V-cycle ----
@@ -2335,15 +2340,15 @@ int poisson_batch_blocks(int64_t nodes, size_t* smem, int* threads, int* blocks,
     PIC_CUDA(cudaGetDevice(&dev));
     PIC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     *threads = nodes >= kBatchHalfNodes * sms ? kBatchHalf : kBatchWhole;
-    *smem = std::max(*smem, *threads / kTileThreads * sizeof(TileMem));
+    *sum_blocks = std::min(sms, kMaxSumBlocks);
+    *smem = std::max({*smem, *threads / kTileThreads * sizeof(TileMem), *sum_blocks * (kSumWarps + 1) * sizeof(double)});
     const void* kernel = batch_kernel(*threads);
     cudaFuncAttributes fa{};  // (grows only: other ensembles may be alive)
     PIC_CUDA(cudaFuncGetAttributes(&fa, kernel));
     if ((int)*smem > fa.maxDynamicSharedSizeBytes)
         PIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem));
     PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, *threads, *smem));
-    *blocks = std::min(per_sm, kBatchWhole / *threads) * sms;
-    *sum_blocks = std::min(sms, kMaxSumBlocks);
+    *blocks = std::min(std::min(per_sm, kBatchWhole / *threads) * sms, kMaxSumBlocks);
     if (*blocks <= 0) return fail(PIC_ERR_CONFIG, "the batched solve does not fit on the device");
     return PIC_OK;
 }
