@@ -137,7 +137,8 @@ constexpr uint32_t kNaOne = 1u << kAxisBits;
 // of those the 32-byte sectors that a warp's additions fall into (about 150 per
 // nanosecond).  So lanes that add to one sector do it with one instruction.
 //
-// Grids whose cells fit into the scratch four words each: a cell's corner sums
+// Grids whose cells fit into the scratch four words each, where they have points
+// enough: a cell's corner sums
 // are a sector, four lanes a point add to it, and k_na_finish_cells gathers a
 // node from its four cells.  Where cells have many points each, blocks add to
 // one of `copies` of the array in turn (additions to one sector wait for each
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(256) k_na_deposit_cells(const pic_point* __res
     }
 }
 
-// Larger grids: a word a node; the two nodes of a cell's row are neighbours,
+// Larger grids, or fewer points: a word a node; the two nodes of a cell's row are neighbours,
 // two lanes a point.
 __global__ void __launch_bounds__(256) k_na_deposit_nodes(const pic_point* __restrict__ pts, int64_t n, int nx, int ny,
                                                           double inv_dx, double inv_dy, unsigned long long* acc) {
@@ -239,11 +240,16 @@ extern "C" int pic_deposit_points_noalloc(const pic_point* dev_points, int64_t n
     const double chrg = -species->charge / epsilon;  // RhoKernel, src/interpolation.cpp:164-170
     const int64_t cells = (int64_t)nx * ny;
     const auto blocks = [](int64_t k) { return (unsigned)((k + 255) / 256); };
-    // Cells where they fit.  Measured, us a call, four scattered additions a point /
-    // nodes in pairs / cells: 4M points on 300 x 280 cells 112 / 81 / 62, on 32 x 32
-    // (16 copies) 628 / 415 / 64, 1M on 300 x 280 40 / 32 / 30; on 700 x 700, too
-    // large for cells, 109 / 81.
-    const bool by_cell = cells * 4 <= kNoAllocMaxNodes;
+    // Cells where they fit and have three points each: clearing and gathering four
+    // words a cell costs more than the additions of fewer.  Measured, us a call, four
+    // scattered additions a point / nodes in pairs / cells: 4M points on 300 x 280
+    // cells 112 / 81 / 62, on 32 x 32 (16 copies) 628 / 415 / 64, 1M on 300 x 280 40 / 32 /
+    // 30; on 700 x 700, too large for cells, 109 / 81.  The three launches alone, without
+    // the host's part of the call: 3,000 points on 362 x 362 5.2 / 5.1 / 6.3, 100,000 6.9 / 6.0 /
+    // 7.0, 300,000 (2.3 a cell) 11.6 / 8.8 / 9.1, 1M 27 / 18 / 16; on 200 x 200 100,000 (2.5)
+    // 7.1 / 6.0 / 6.1, 200,000 10.0 / 7.9 / 7.2; on 100 x 100 20,000 5.3 / 5.0 / 5.1, 30,000 6.0 /
+    // 5.3 / 5.2.
+    const bool by_cell = cells * 4 <= kNoAllocMaxNodes && n >= 3 * cells;
     int copies = 1;  // up to 16, while the cells have 64 points each a copy
     while (by_cell && copies < 16 && cells * 8 * copies <= kNoAllocMaxNodes && n >= cells * 128 * copies) copies *= 2;
     const int64_t words = by_cell ? cells * 4 * copies : nodes;
