@@ -972,8 +972,10 @@ __device__ __forceinline__ uint32_t scan_value(const uint32_t* in, int64_t t) {
     return CAP ? cell_capacity(in[t]) : in[t];
 }
 
+// With CAP counters[3] collects the total, which may be beyond 32 bits.
 template <bool CAP>
-__global__ void __launch_bounds__(256) k_scan_partials(const uint32_t* in, int64_t n, uint32_t* partials) {
+__global__ void __launch_bounds__(256) k_scan_partials(const uint32_t* in, int64_t n, uint32_t* partials,
+                                                       unsigned long long* counters) {
     __shared__ uint32_t red[8];
     const int64_t base = (int64_t)blockIdx.x * kScanTile;
     uint32_t s = 0;
@@ -989,6 +991,7 @@ __global__ void __launch_bounds__(256) k_scan_partials(const uint32_t* in, int64
         uint32_t t = 0;
         for (int w = 0; w < 8; ++w) t += red[w];
         partials[blockIdx.x] = t;
+        if (CAP) atomicAdd(counters + 3, (unsigned long long)t);
     }
 }
 
@@ -1307,19 +1310,28 @@ __global__ void k_plasma_generate(PlasmaArgs P, const uint32_t* __restrict__ den
 
 inline unsigned grid1d(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
+constexpr unsigned long long kMaxSlots = 0xF0000000ull;  // of a species
+
 // out[0..n] = exclusive scan of in (CAP: of cell capacities); returns the
-// total through *total when not null (synchronises).
+// total through *total when not null (synchronises).  Capacities beyond the
+// 32-bit slot indices are an error.
 template <bool CAP>
 int scan_cells(pic_ctx* c, Species& sp, const uint32_t* in, uint32_t* out, uint32_t* total) {
     const int64_t n = c->ncells;
     const int nparts = (int)((n + kScanTile - 1) / kScanTile);
-    k_scan_partials<CAP><<<nparts, 256, 0, c->stream>>>(in, n, c->scan_partials);
+    if (CAP) PIC_CUDA(cudaMemsetAsync(sp.counters + 3, 0, 8, c->stream));
+    k_scan_partials<CAP><<<nparts, 256, 0, c->stream>>>(in, n, c->scan_partials, sp.counters);
     k_scan_apply<CAP><<<nparts, 256, 0, c->stream>>>(in, n, c->scan_partials, out, sp.counters);
     c->launches += 2;
     PIC_CUDA(cudaGetLastError());
     if (total) {
-        PIC_CUDA(cudaMemcpyAsync(total, out + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+        unsigned long long t = 0;
+        if (CAP) PIC_CUDA(cudaMemcpyAsync(&t, sp.counters + 3, 8, cudaMemcpyDeviceToHost, c->stream));
+        else PIC_CUDA(cudaMemcpyAsync(&t, out + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
         PIC_CUDA(cudaStreamSynchronize(c->stream));
+        if (t > kMaxSlots && CAP)
+            return fail(PIC_ERR_CAPACITY, "a species holds at most 4.0e9 particle slots (32-bit indices)");
+        *total = (uint32_t)t;
     }
     return PIC_OK;
 }
@@ -1492,11 +1504,11 @@ static int list_alloc(LooseList& L, uint32_t cap, uint32_t* count) {
     cudaFree(L.vz);
     cudaFree(L.cell);
     L = LooseList{};
+    L.count = count;  // (a list without room is an empty one to the kernels)
     PIC_CUDA(cudaMalloc(&L.a, (size_t)cap * sizeof(float4)));
     PIC_CUDA(cudaMalloc(&L.vz, (size_t)cap * sizeof(float)));
     PIC_CUDA(cudaMalloc(&L.cell, (size_t)cap * sizeof(uint32_t)));
     L.cap = cap;
-    L.count = count;
     return PIC_OK;
 }
 
@@ -1591,7 +1603,7 @@ static int grow_store(pic_ctx* c, int s, int64_t capacity) {
     if (capacity <= sp.capacity && sp.store) return PIC_OK;
     // multiples of 64 slots keep both buffers' float4 arrays 256-byte aligned
     capacity = (capacity + 63) & ~(int64_t)63;
-    if (capacity > (int64_t)0xF0000000ll)
+    if (capacity > (int64_t)kMaxSlots)
         return fail(PIC_ERR_CAPACITY, "a species holds at most 4.0e9 particle slots (32-bit indices)");
     float* store = nullptr;
     PIC_CUDA(cudaMalloc(&store, (size_t)capacity * 2 * 5 * sizeof(float)));
@@ -1620,7 +1632,7 @@ static int grow_store(pic_ctx* c, int s, int64_t capacity) {
 static int grow_lists(pic_ctx* c, int s) {
     Species& sp = c->sp[s];
     const uint32_t lc = list_capacity(sp.capacity);
-    if (lc <= sp.ovf.cap) return PIC_OK;
+    if (lc <= std::min({sp.ovf.cap, sp.loose[0].cap, sp.loose[1].cap})) return PIC_OK;
     PIC_CUDA(cudaStreamSynchronize(c->stream));
     PIC_TRY(list_alloc(sp.ovf, lc, sp.list_counts + kOvf));
     PIC_TRY(list_alloc(sp.loose[0], lc, sp.list_counts + kLoose0));
@@ -1750,32 +1762,54 @@ int particles_import_staging(pic_ctx* c, int64_t n, PointRec** dev_recs) {
     return PIC_OK;
 }
 
+// Leaves a species without particles, and without room for any: after its
+// buffers were given up and larger ones, or larger lists, could not be had.
+static int drop_particles(pic_ctx* c, Species& sp) {
+    const size_t bytes = (size_t)c->ncells * 4;
+    cudaGetLastError();
+    PIC_CUDA(cudaMemsetAsync(sp.base, 0, bytes + 4, c->stream));
+    for (int b = 0; b < 2; ++b) {
+        PIC_CUDA(cudaMemsetAsync(sp.front[b], 0, bytes, c->stream));
+        PIC_CUDA(cudaMemsetAsync(sp.back[b], 0, bytes, c->stream));
+    }
+    PIC_CUDA(cudaStreamSynchronize(c->stream));
+    sp.acc_fresh = false;
+    return PIC_OK;
+}
+
 // Installs a fresh layout from sp.cnt (particles per cell): base from the
 // cell capacities, growing the buffers when needed.  The current buffer's
-// contents are dropped.
+// contents are dropped, unless the counts are refused.
 static int fresh_layout(pic_ctx* c, int s) {
     Species& sp = c->sp[s];
     uint32_t total = 0;
-    PIC_TRY(scan_cells<true>(c, sp, sp.cnt, sp.base, &total));
-    PIC_CUDA(cudaMemsetAsync(sp.list_counts, 0, 4 * sizeof(uint32_t), c->stream));
-    sp.lcur = 0;
-    sp.flags_pending = false;
-    sp.loose_count = 0u;
-    sp.ppc = mean_count(c, total);
-    if ((int64_t)total > sp.capacity) {
-        PIC_CUDA(cudaStreamSynchronize(c->stream));
-        cudaFree(sp.store);
-        sp.store = nullptr;
-        sp.capacity = 0;
-        PIC_TRY(grow_store(c, s, total));
-    }
-    PIC_TRY(grow_lists(c, s));
+    PIC_TRY(scan_cells<true>(c, sp, sp.cnt, sp.base_next, &total));
     unsigned long long flags[2] = {0, 0};
     PIC_CUDA(cudaMemcpyAsync(flags, sp.counters, sizeof(flags), cudaMemcpyDeviceToHost, c->stream));
     PIC_CUDA(cudaStreamSynchronize(c->stream));
     if (flags[1]) {
         PIC_CUDA(cudaMemsetAsync(sp.counters + 1, 0, 8, c->stream));
         return fail(PIC_ERR_CAPACITY, "a cell exceeds the per-cell particle limit");
+    }
+    std::swap(sp.base, sp.base_next);
+    PIC_CUDA(cudaMemsetAsync(sp.list_counts, 0, 4 * sizeof(uint32_t), c->stream));
+    sp.lcur = 0;
+    sp.flags_pending = false;
+    sp.loose_count = 0u;
+    sp.ppc = mean_count(c, total);
+    int st = PIC_OK;
+    if ((int64_t)total > sp.capacity) {
+        PIC_CUDA(cudaStreamSynchronize(c->stream));
+        cudaFree(sp.store);
+        sp.store = nullptr;
+        sp.capacity = 0;
+        st = grow_store(c, s, total);
+    }
+    if (st == PIC_OK) st = grow_lists(c, s);
+    if (st != PIC_OK) {
+        const std::string why = pic_last_error();
+        PIC_TRY(drop_particles(c, sp));
+        return fail(st, why);
     }
     return PIC_OK;
 }
