@@ -259,7 +259,7 @@ def measured_peaks():
 
 
 def ncu_traffic_per_particle():
-    """Per-particle DRAM bytes of the scatter pass from the committed ncu
+    """Per-particle DRAM bytes of a push from the committed ncu
     summary (profiles/traffic.txt), or None."""
     p = os.path.join(ROOT, "profiles", "traffic.txt")
     if not os.path.exists(p):
@@ -373,7 +373,7 @@ def run_ours(args, rank, world, local_rank):
     avg_n = n_part / 2
     achieved = BYTES_PUSH_PASS * avg_n / (push_ms * 1e-3) / 1e9
     traffic_pp, traffic_src = ncu_traffic_per_particle()
-    roofline = {"kernel": "k_cells<kPush> (gather + Boris + binning + fused deposit, one pass)",
+    roofline = {"kernel": "k_cells<kPush> + k_cells<kArrivals> (gather + Boris + binning + deposit)",
                 "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_kind": f"{peak_kind} hbm_gbs",
                 "bytes_per_particle": BYTES_PUSH_PASS,

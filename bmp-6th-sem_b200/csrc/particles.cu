@@ -16,8 +16,9 @@
 // that moved in), with a free gap between them.
 //
 // One push of a species is ONE pass over its particles (k_cells<kPush>).  A
-// warp works on a few neighbouring cells at a time, 4, 8 or 16 lanes a cell;
-// it gathers E and Bz, pushes, and
+// warp works on a few neighbouring cells at a time, 4, 8 or 16 lanes a cell
+// (32 where a cell is far fuller than its neighbours); it gathers E and Bz,
+// pushes, and
 //   * writes a particle that stays in its cell to the front of the cell's
 //     slots in the other buffer, at its rank among the cell's stayers
 //     (ballot + popc: no atomics), and adds its deposit to per-lane integer
@@ -38,7 +39,7 @@
 // read + 20 B written.
 //
 // Measured on a B200, push + arrivals, electrons / Ar+: the 1024^2 workload
-// (1.15e8 particles each) 1.26 / 0.88 ms (with a warp a cell, 32-lane chunks
+// (1.15e8 particles each) 1.26 / 0.87 ms (with a warp a cell, 32-lane chunks
 // and the movers deposited one by one: 1.83 / 1.17 ms); 512^2 at 64 a cell
 // 0.23 / 0.14 ms (0.28 / 0.18); 64 grids of 128^2 .. 384^2 at 32 a cell 4.2 ms
 // both (8.2 ms).  The Ar+ pass runs at 5.2 TB/s of reads and writes, 0.8 of a
@@ -481,8 +482,8 @@ struct CellMeta {
 };
 
 // Particles that left their cell wait in a per-warp queue in shared memory
-// and are placed 32 at a time (all lanes busy): cell bookkeeping, deposit,
-// grouping by target cell (match.any), one slot reservation per group, store.
+// and are placed 32 at a time (all lanes busy): cell bookkeeping, a slot
+// reserved by one atomic each, store.
 constexpr int kQueue = 96;  // 31 waiting and a chunk of 64
 
 struct MoverQueue {
@@ -793,7 +794,7 @@ __device__ __forceinline__ void cells_body(const KArgs& A, Tile T, uint32_t tile
 }
 
 // The tiles of the tile shapes 1, 2 and 3 (256 cells), and the two that shape
-// 0 chooses from (auto_tile).
+// 0 chooses from (pick_tile).
 constexpr int kNumTileShapes = 4;
 constexpr int kNumTiles = 5;
 constexpr Tile kTile[kNumTiles] = {{5, 0}, {8, 0}, {7, 1}, {4, 4}, {6, 0}};
@@ -1428,7 +1429,8 @@ int pick_tile(int shape, double ppc, int64_t tiles64) {
 // Lanes a cell of a push.  Few lanes: a warp's set has more cells, so the
 // per-set work (metadata, reduction, REDs) is shared by more of them and
 // sparse cells leave fewer lanes idle; many lanes: longer contiguous runs an
-// access.  Measured, electron + ion push of a 512^2 grid in us with 4 / 8 /
+// access.  (By the mean: tiles with cells far fuller than the rest see to
+// themselves, crowded().)  Measured, electron + ion push of a 512^2 grid in us with 4 / 8 /
 // 16 lanes: 4 particles a cell 100 / 114 / 169, 8: 118 / 126 / 174, 16: 168 /
 // 162 / 189, 32: 254 / 230 / 240, 48: 355 / 313 / 309, 64: 430 / 374 / 366.
 int pick_lanes(double ppc) { return ppc >= 48.0 ? 16 : (ppc >= 12.0 ? 8 : 4); }

@@ -108,7 +108,7 @@ struct ParticleSoA {
 };
 
 // Particles held outside the cell layout (a mover that found its target
-// cell full, or one that jumped more than one cell): state plus target cell.
+// cell full, a new particle of a source): state plus target cell.
 struct LooseList {
     float4* a = nullptr;
     float* vz = nullptr;
@@ -304,7 +304,7 @@ int particles_export_state(pic_ctx* c, int s, void* dev, int64_t n);
 int particles_deposit(pic_ctx* c, int s);       // fresh deposit of current positions
 // acc -> final/energy mesh, rho += (from zero with zero_rho) of species s0 .. s0 + ns - 1
 int particles_flush(pic_ctx* c, int s0, int ns, bool zero_rho);
-int particles_push(pic_ctx* c, int s);          // pass1 + scan + pass2 (+deposit)
+int particles_push(pic_ctx* c, int s);          // push, deposit of the arrivals, side lists
 int particles_count(pic_ctx* c, int s, int64_t* n);
 int particles_bin_counts(pic_ctx* c, int s, int32_t* dev_counts);
 // batched particle phases over an ensemble's contexts (particles.cu)

@@ -25,9 +25,11 @@
 // 32 nodes: those that start in its band.  phi, r and z of other blocks are
 // read after a barrier and past L1.
 //
-// alpha and beta are the multi-kernel solve's bit for bit (so are then the
-// iterates, and a run does not depend on which of the two solved it): r.z is
-// summed in the order of k_mg_up's tiles, p.A p in that of k_pcg_pq's blocks.
+// alpha and beta are the multi-kernel solve's bit for bit, and so is every
+// iterate: r.z is summed in the order of k_mg_up's tiles, p.A p in that of
+// k_pcg_pq's blocks.  |r|^2 and |b|^2, which only decide when to stop, are sums of
+// the blocks' own: the two solvers end an iteration apart if a residual comes
+// within some 1e-15 of the tolerance, and else give the same potential.
 // A warp sums what one of their warps sums and stores it in every block, which
 // then finishes the sum as reduce_finalize does.  That costs two cluster
 // barriers an iteration more than sums of the blocks' own (of 129^2 nodes: 6 in
@@ -113,8 +115,8 @@ __device__ __forceinline__ void cluster_barrier() {
 }
 
 struct ClShared {
-    double red[3][kClThreads / 32];
-    double part[3][kClBlocks][3];            // every block's partial sums, three in turn
+    double red[2][kClThreads / 32];
+    double part[3][kClBlocks][2];            // every block's partial sums, three in turn
     int start[kClMaxLevels + 1][kClBlocks + 1];  // first row of each level that each block owns
 };
 
@@ -136,7 +138,7 @@ struct ClBlock {
         return j < 0 ? j + GY : j;
     }
 
-    // Sums of up to three values over the cluster (in place), the same bits in
+    // Sums of one or two values over the cluster (in place), the same bits in
     // every thread of every block; also a cluster barrier.  Each block stores
     // its partials in every block's table before the barrier (no remote read
     // after it).

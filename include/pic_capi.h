@@ -401,9 +401,11 @@ int pic_ensemble_info(pic_ensemble* ens, int* graph_active, int* tile_shape, int
 /* ---- Poisson controls -------------------------------------------------- */
 int pic_set_poisson(pic_ctx* ctx, int solver, int warm_start, double tol, int maxit);
 /* (no reference counterpart) enable = 0: run the PCG iterations as direct
- * launches with one host synchronisation per iteration instead of one CUDA
- * graph per solve (same kernels, same results; slower).  For profilers that
- * do not follow the kernels of a graph's conditional node.  Default 1. */
+ * launches with one host synchronisation per iteration, instead of one CUDA
+ * graph per solve (the same kernels) or, on grids of up to 14,000 nodes, one
+ * launch of a thread-block cluster (another kernel; the same iterates, bit for
+ * bit).  Slower.  For profilers that do not follow the kernels of a graph's
+ * conditional node.  Default 1. */
 int pic_set_poisson_graph(pic_ctx* ctx, int enable);
 /* Iterations, achieved relative residual and device milliseconds of the most
  * recent solve. */
