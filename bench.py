@@ -444,7 +444,7 @@ def kernel_rooflines(w, counts, ev, pois_ms, iters, phases, peak, peak_kind):
     for s, name in ((0, "electrons"), (1, "Ar+")):
         ms = sum((e[4].elapsed_time(e[3]) if s == 1 else e[2].elapsed_time(e[4])) for e in ev) / steps
         gbs = BYTES_PUSH_PASS * counts[s] / (ms * 1e-3) / 1e9
-        out.append({"kernel": f"k_cells<kPush> {name} pass (+ k_fixup)", "ms": ms,
+        out.append({"kernel": f"k_cells<kPush> {name} pass (+ k_cells<kArrivals>, k_fixup)", "ms": ms,
                     "bytes": BYTES_PUSH_PASS * counts[s], "achieved_GBs": gbs, "frac": gbs / peak})
     fl = phases["flush"]
     if fl["calls_per_step"]:
